@@ -9,8 +9,18 @@ namespace wust {
 constexpr int kFactorTile = 48;
 // padded interior size of a working page (multiple of the output tile)
 constexpr size_t factor_pad(int ny) { return ((size_t)(ny - 2) + kFactorTile - 1) / kFactorTile * kFactorTile; }
+constexpr int kFlowBlock = 16;            // Gauss-Jordan block of the dataflow kernel
+constexpr int kFlowMaxTiles = 12;         // tiles per page edge of the dataflow kernel: 12 x 12 <= 148 CTAs
 // two ping-pong working pages + barrier/status words
-constexpr size_t factor_scratch_bytes_for(int ny) { return 2 * factor_pad(ny) * factor_pad(ny) * 8 + 256; }
+constexpr size_t factor_pages_bytes(int ny) { return 2 * factor_pad(ny) * factor_pad(ny) * 8 + 256; }
+// per step: the row and column panels and the inverse pivot block in 16-byte words
+constexpr size_t factor_flow_bytes(int ny) {
+    return ((size_t)(ny - 2) + kFlowBlock - 1) / kFlowBlock * kFlowBlock * 16 * (2 * factor_pad(ny) + kFlowBlock) + 256;
+}
+constexpr size_t factor_scratch_bytes_for(int ny) {
+    return factor_pad(ny) <= (size_t)kFlowMaxTiles * kFactorTile && factor_flow_bytes(ny) > factor_pages_bytes(ny)
+               ? factor_flow_bytes(ny) : factor_pages_bytes(ny);
+}
 size_t factor_scratch_bytes(int ny);
 // host_status (nullable, int[3]): {1+bad page, pivot, barrier timeout site};
 // when non-null the call synchronizes the stream.  Pages [j0, j1) are
