@@ -53,3 +53,30 @@ def test_factor_reports_a_singular_page(ny, row):
     with pytest.raises(WustError, match=rf"block 1 is singular at pivot {row}"):
         decompBlockLU(*_device(bad))
     assert np.array_equal(decompBlockLU(*_device(coefs)).cpu().numpy(), good)
+
+
+# one interior row; odd and even column lengths (the parity of a page column's first byte); the largest column of the
+# widest shape, the first beyond it, and the first that takes a launch per column step
+@pytest.mark.parametrize("ny,nx,S", [(3, 3, 1), (3, 5, 3), (18, 7, 5), (19, 6, 2), (64, 9, 13), (97, 8, 1), (194, 5, 40),
+                                     (195, 5, 41), (578, 4, 30), (642, 4, 20), (770, 4, 3), (771, 4, 3)])
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_sweeps_match_the_fp64_substitution(ny, nx, S, adjoint):
+    """The substitutions on given pages, sources on the border included, from views on 16 and on 8 bytes."""
+    import torch
+    from oracle import helmholtz_fp64 as o
+    from waveforminversionust_b200.solver import applyBlockLU, decompBlockLU
+    coefs = _blocks(ny, nx)
+    dev = _device(coefs)
+    inv = decompBlockLU(*dev)
+    g = np.random.default_rng(S)
+    src = (g.standard_normal((ny, nx, S)) + 1j * g.standard_normal((ny, nx, S))).astype(np.complex64)
+    sides = [dev[i] for i in (0, 1, 2, 6, 7, 8)]
+    u = applyBlockLU(src, *sides, inv, adjoint).cpu().numpy()
+    want = o.block_lu_apply(src.astype(np.complex128), {n: coefs[n].astype(np.complex64) for n in NAMES},
+                            inv.cpu().numpy().astype(np.complex128), adjoint)
+    # 2 (nx - 1) products of n terms in 32 bits, rounded like a random walk: 2e-5 leaves an order of magnitude
+    assert np.linalg.norm(u - want) < 2e-5 * np.linalg.norm(want)
+    shifted = torch.empty(nx * ny * ny + 1, dtype=torch.complex64, device="cuda")[1:].view(nx, ny, ny)
+    shifted.copy_(inv.permute(2, 1, 0))
+    v = applyBlockLU(src, *sides, shifted.permute(2, 1, 0), adjoint).cpu().numpy()
+    assert np.linalg.norm(v - want) < 2e-5 * np.linalg.norm(want)

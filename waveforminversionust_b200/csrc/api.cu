@@ -152,7 +152,7 @@ struct wust_solver {
     uint8_t *tc_afwd = nullptr, *tc_aadj = nullptr, *tc_b = nullptr;
     float *tc_part = nullptr;
     unsigned *tc_sync = nullptr;
-    int *tc_err = nullptr;
+    int *sweep_err = nullptr;
     TcSweepGeom tc_geom{};
     // column-chunked tensor-core sweeps (TF32 profile, default): packed
     // -Lambda_c pages, per-group B chunks, chunk and boundary states, counters
@@ -169,7 +169,7 @@ struct wust_solver {
     bool bf16_all = false;
     uint8_t *tc_afwd16 = nullptr, *tc_aadj16 = nullptr, *ck_lpack16 = nullptr;
     TcChunkBuffers chunk_buffers() const {
-        return TcChunkBuffers{ck_lpack, ck_b, ck_lpack16, ck_z, ck_sb, ck_edges, ck_sync, tc_err};
+        return TcChunkBuffers{ck_lpack, ck_b, ck_lpack16, ck_z, ck_sb, ck_edges, ck_sync, sweep_err};
     }
     // Newton-Schulz factorization (TF32 profile)
     void *ns_scratch = nullptr;
@@ -222,7 +222,7 @@ static void free_solver(wust_solver *s) {
     void *ptrs[] = {s->vel, s->atten, s->exi, s->eyi, s->mult, s->status, s->invT, s->fscratch, s->u, s->lam,
                     s->tmp, s->work, s->x64, s->x64b, s->w9f, s->w9a, s->r32, s->d32, s->rnorm2, s->bnorm2, s->dnorm2, s->xnorm2, s->tx_lin, s->rx_lin,
                     s->rx_at, s->Yd, s->maskd, s->resid, s->scale, s->loss_src, s->grad, s->dir, s->ret_u,
-                    s->stage_d, s->stage_c, s->tc_afwd, s->tc_aadj, s->tc_b, s->tc_part, s->tc_sync, s->tc_err, s->ns_scratch,
+                    s->stage_d, s->stage_c, s->tc_afwd, s->tc_aadj, s->tc_b, s->tc_part, s->tc_sync, s->sweep_err, s->ns_scratch,
                     s->ck_lpack, s->ck_b, s->ck_z, s->ck_sb, s->ck_edges, s->ck_sync,
                     s->tc_afwd16, s->tc_aadj16, s->ck_lpack16};
     for (void *p : ptrs) dfree(p);
@@ -376,9 +376,9 @@ static void run_sweep(wust_solver *s, const SrcView &src, int S, bool adjoint, f
                            s->chunk_buffers(), src, S, adjoint, out, bf16, s->st);
         else
             tc_sweep_solve(s->coefs64(), s->tc_afwd, s->tc_aadj, s->tc_geom, src, S, adjoint, out, s->tc_b,
-                           s->tc_part, s->tc_sync, s->tc_err, s->st);
+                           s->tc_part, s->tc_sync, s->sweep_err, s->st);
     } else {
-        sweep_solve(s->coefs64(), s->invT, src, S, adjoint, out, s->tmp, s->st);
+        sweep_solve(s->coefs64(), s->invT, src, S, adjoint, out, s->tmp, s->sweep_err, s->st, s->max_ctas);
     }
     WUST_CUDA(cudaEventRecord(s->sw_ev[1], s->st));
     WUST_CUDA(cudaEventSynchronize(s->sw_ev[1]));
@@ -388,14 +388,13 @@ static void run_sweep(wust_solver *s, const SrcView &src, int S, bool adjoint, f
     ++s->sweeps;
 }
 
-static void check_tc_err(wust_solver *s) {
-    if (!s->tc_err) return;
+static void check_sweep_err(wust_solver *s) {
     int e = 0;
-    WUST_CUDA(cudaMemcpyAsync(&e, s->tc_err, sizeof(int), cudaMemcpyDeviceToHost, s->st));
+    WUST_CUDA(cudaMemcpyAsync(&e, s->sweep_err, sizeof(int), cudaMemcpyDeviceToHost, s->st));
     WUST_CUDA(cudaStreamSynchronize(s->st));
     if (e) {
-        WUST_CUDA(cudaMemsetAsync(s->tc_err, 0, sizeof(int), s->st));
-        fail(WUST_ERR_DEVICE_TIMEOUT, "tensor-core pipeline wait expired (code %d)", e);
+        WUST_CUDA(cudaMemsetAsync(s->sweep_err, 0, sizeof(int), s->st));
+        fail(WUST_ERR_DEVICE_TIMEOUT, "sweep pipeline wait expired (code %d)", e);
     }
 }
 
@@ -424,7 +423,10 @@ static void solve_into(wust_solver *s, const SrcView &src, int S, bool adjoint, 
     s->last_refine_iters = 0;
     s->last_residual = -1;
     s->last_error_est = -1;
-    if (s->precision == WUST_PRECISION_C64) return;
+    if (s->precision == WUST_PRECISION_C64) {
+        check_sweep_err(s);
+        return;
+    }
     std::vector<double> rn(S), rn_prev(S), bn(S), dn(S), xn(S);
     // BF16 corrections (half the operand bytes) as long as they contract the
     // residual at least kBf16Contraction-fold per correction; a weaker step
@@ -441,7 +443,7 @@ static void solve_into(wust_solver *s, const SrcView &src, int S, bool adjoint, 
     WUST_CUDA(cudaMemcpyAsync(rn.data(), s->rnorm2, S * sizeof(double), cudaMemcpyDeviceToHost, st));
     WUST_CUDA(cudaMemcpyAsync(bn.data(), s->bnorm2, S * sizeof(double), cudaMemcpyDeviceToHost, st));
     WUST_CUDA(cudaStreamSynchronize(st));
-    check_tc_err(s);
+    check_sweep_err(s);
     for (int k = 1;; ++k) {
         if (k > s->refine_max)
             fail(WUST_ERR_NOT_CONVERGED, "refinement did not reach %.1e after %d correction solves (estimate %.3e)",
@@ -463,7 +465,7 @@ static void solve_into(wust_solver *s, const SrcView &src, int S, bool adjoint, 
         WUST_CUDA(cudaMemcpyAsync(dn.data(), s->dnorm2, S * sizeof(double), cudaMemcpyDeviceToHost, st));
         WUST_CUDA(cudaMemcpyAsync(xn.data(), s->xnorm2, S * sizeof(double), cudaMemcpyDeviceToHost, st));
         WUST_CUDA(cudaStreamSynchronize(st));
-        check_tc_err(s);
+        check_sweep_err(s);
         double worst_err = 0, worst_res = 0, worst_rho = 0;
         for (int q = 0; q < S; ++q) {
             if (!(std::isfinite(rn[q]) && std::isfinite(dn[q]) && std::isfinite(xn[q])))
@@ -578,18 +580,23 @@ int wust_apply_block_lu(const wust_c64 *src, int Ny, int Nx, int n_src, const wu
         co.Ud = (const float2 *)Ud; co.Ul = (const float2 *)Ul; co.Uu = (const float2 *)Uu;
         co.ny = Ny; co.nx = Nx;
         float2 *tmp = nullptr;
-        WUST_CUDA(cudaMalloc(&tmp, sizeof(float2) * (size_t)Ny * n_src));
+        const size_t tmp_n = (size_t)Ny * n_src;
+        int err = 0;
+        WUST_CUDA(cudaMalloc(&tmp, sizeof(float2) * (tmp_n + 1)));    // and the word of an expired wait
         SrcView sv{};
         sv.mode = SRC_DENSE;
         sv.dense = (const float2 *)src;
         try {
-            sweep_solve(co, (const float2 *)invT, sv, n_src, adjoint != 0, (float2 *)u, tmp, st);
+            WUST_CUDA(cudaMemsetAsync(tmp + tmp_n, 0, sizeof(float2), st));
+            sweep_solve(co, (const float2 *)invT, sv, n_src, adjoint != 0, (float2 *)u, tmp, (int *)(tmp + tmp_n), st);
+            WUST_CUDA(cudaMemcpyAsync(&err, tmp + tmp_n, sizeof(int), cudaMemcpyDeviceToHost, st));
             WUST_CUDA(cudaStreamSynchronize(st));
         } catch (...) {
             cudaFree(tmp);
             throw;
         }
         cudaFree(tmp);
+        if (err) fail(WUST_ERR_DEVICE_TIMEOUT, "block sweep wait expired (code %d)", err);
     });
 }
 
@@ -675,6 +682,8 @@ int wust_solver_create(wust_solver **out, const wust_solver_options *o, const do
         s->grad = dalloc<double>(N);
         s->dir = dalloc<double>(N);
         s->rx_at = dalloc<int32_t>(N);
+        s->sweep_err = dalloc<int>(4);
+        WUST_CUDA(cudaMemset(s->sweep_err, 0, 4 * sizeof(int)));
         if (s->precision != WUST_PRECISION_C64) {
             s->x64 = dalloc<double2>(F);
             s->x64b = dalloc<double2>(F);
@@ -701,8 +710,6 @@ int wust_solver_create(wust_solver **out, const wust_solver_options *o, const do
                 s->ns_g = ns_geom(ny, capped(ns_max_ctas()), s->max_ctas == 0);
                 if (s->ns_g.ks > 0) WUST_CUDA(cudaMalloc(&s->ns_scratch, s->ns_g.scratch_bytes));
             }
-            s->tc_err = dalloc<int>(4);
-            WUST_CUDA(cudaMemset(s->tc_err, 0, 4 * sizeof(int)));
             if (s->sweep_method == WUST_SWEEP_DEFAULT) {
                 s->ck_geom = tc_chunk_geom(ny, nx, capped(tc_chunk_max_ctas()), s->chunk_count);
                 s->use_chunks = s->ck_geom.C >= 2;   // one chunk: the sequential kernel is faster

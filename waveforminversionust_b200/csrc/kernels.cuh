@@ -32,9 +32,11 @@ void factor_launch(const Coefs<float2> &co, float2 *invT, void *scratch, size_t 
 int barrier_selftest(double timeout_s, int *site_out);
 
 // ---- sweep.cu --------------------------------------------------------------
-// u (ny*nx*S) is overwritten; tmp needs ny*S elements.
+// u (ny*nx*S) is overwritten; tmp needs ny*S elements; *err (device, zero
+// before the call) receives the site of an expired device wait.  max_ctas >
+// 0: CTAs that may run at once (a solver confined to part of the GPU).
 void sweep_solve(const Coefs<float2> &co, const float2 *invT, const SrcView &src, int S, bool adjoint,
-                 float2 *u, float2 *tmp, cudaStream_t st);
+                 float2 *u, float2 *tmp, int *err, cudaStream_t st, int max_ctas = 0);
 
 // ---- tcsweep.cu (tensor-core sweeps, TF32 inputs) --------------------------
 struct TcSweepGeom {
