@@ -268,6 +268,15 @@ int wust_ncg_project(wust_solver *s, double *c, const double *direction, double 
 int wust_dtft(const double *time_s, int n_time, const double *frequencies_hz, int n_f, const void *rf, int rf_is_double,
               int n_rx, int n_tx, const uint8_t *active, wust_c64 *Y, void *stream);
 
+/* wust_dtft for callers that keep device memory of their own: workspace is
+ * device memory of at least wust_dtft_workspace_bytes(n_time, n_f) bytes on a
+ * 256-byte boundary, used until the call returns (NULL: the call allocates and
+ * frees it, as wust_dtft does). */
+size_t wust_dtft_workspace_bytes(int n_time, int n_f);
+int wust_dtft_ws(const double *time_s, int n_time, const double *frequencies_hz, int n_f, const void *rf, int rf_is_double,
+                 int n_rx, int n_tx, const uint8_t *active, wust_c64 *Y, void *workspace, size_t workspace_bytes,
+                 void *stream);
+
 /* RF simulation of wust_simulate.m:1-87 (its 'native-batch' and
  * 'matlab-serial' backends, which run k-Wave's 2-D first-order k-space solver
  * per transmitter): linear acoustics, scalar density rho0, no absorption, a

@@ -1121,8 +1121,13 @@ int wust_ncg_project(wust_solver *s, double *c, const double *direction, double 
     });
 }
 
-int wust_dtft(const double *time_s, int n_time, const double *frequencies_hz, int n_f, const void *rf, int rf_is_double,
-              int n_rx, int n_tx, const uint8_t *active, wust_c64 *Y, void *stream) {
+size_t wust_dtft_workspace_bytes(int n_time, int n_f) {
+    return n_time < 1 || n_f < 1 ? 0 : dtft_workspace_bytes(n_time, n_f);
+}
+
+int wust_dtft_ws(const double *time_s, int n_time, const double *frequencies_hz, int n_f, const void *rf, int rf_is_double,
+                 int n_rx, int n_tx, const uint8_t *active, wust_c64 *Y, void *workspace, size_t workspace_bytes,
+                 void *stream) {
     return guarded([&] {
         if (!time_s || !frequencies_hz || !rf || !active || !Y) fail(WUST_ERR_INVALID_INPUT, "dtft arguments missing");
         if (n_time < 2 || n_f < 1 || n_rx < 1 || n_tx < 1) fail(WUST_ERR_INVALID_INPUT, "Invalid sample times");
@@ -1136,28 +1141,32 @@ int wust_dtft(const double *time_s, int n_time, const double *frequencies_hz, in
         for (int k = 0; k < n_f; ++k)
             if (!(std::isfinite(frequencies_hz[k]) && frequencies_hz[k] > 0 && frequencies_hz[k] < 0.5 / dt))
                 fail(WUST_ERR_INVALID_INPUT, "Frequency outside saved Nyquist");
+        const size_t need = dtft_workspace_bytes(n_time, n_f);
+        if (workspace && (workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0))
+            fail(WUST_ERR_INVALID_INPUT, "dtft workspace of %zu bytes on 256 required", need);
         cudaStream_t st = static_cast<cudaStream_t>(stream);
-        double *t_d = nullptr, *f_d = nullptr;
-        double2 *K = nullptr;
-        int *bad = nullptr;
-        WUST_CUDA(cudaMallocAsync(&t_d, sizeof(double) * n_time, st));
-        WUST_CUDA(cudaMallocAsync(&f_d, sizeof(double) * n_f, st));
-        WUST_CUDA(cudaMallocAsync(&K, sizeof(double2) * (size_t)n_time * n_f, st));
-        WUST_CUDA(cudaMallocAsync(&bad, sizeof(int), st));
-        WUST_CUDA(cudaMemcpyAsync(t_d, time_s, sizeof(double) * n_time, cudaMemcpyHostToDevice, st));
-        WUST_CUDA(cudaMemcpyAsync(f_d, frequencies_hz, sizeof(double) * n_f, cudaMemcpyHostToDevice, st));
-        WUST_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), st));
-        dtft_launch(t_d, f_d, n_time, n_f, dt, rf, rf_is_double != 0, n_rx, n_tx, active, K,
-                    reinterpret_cast<float2 *>(Y), bad, st);
-        int h_bad = 0;
+        // freed on every way out
+        struct Own {
+            void *p = nullptr;
+            cudaStream_t st;
+            ~Own() { if (p) cudaFreeAsync(p, st); }
+        } own{nullptr, st};
+        if (!workspace) {
+            WUST_CUDA(cudaMallocAsync(&own.p, need, st));
+            workspace = own.p;
+        }
+        int *bad = nullptr, h_bad = 0;
+        dtft_launch(time_s, frequencies_hz, n_time, n_f, dt, rf, rf_is_double != 0, n_rx, n_tx, active, workspace,
+                    reinterpret_cast<float2 *>(Y), &bad, st);
         WUST_CUDA(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
-        WUST_CUDA(cudaFreeAsync(t_d, st));
-        WUST_CUDA(cudaFreeAsync(f_d, st));
-        WUST_CUDA(cudaFreeAsync(K, st));
-        WUST_CUDA(cudaFreeAsync(bad, st));
         WUST_CUDA(cudaStreamSynchronize(st));
         if (h_bad) fail(WUST_ERR_INVALID_INPUT, "Nonfinite RF on an active channel");
     });
+}
+
+int wust_dtft(const double *time_s, int n_time, const double *frequencies_hz, int n_f, const void *rf, int rf_is_double,
+              int n_rx, int n_tx, const uint8_t *active, wust_c64 *Y, void *stream) {
+    return wust_dtft_ws(time_s, n_time, frequencies_hz, n_f, rf, rf_is_double, n_rx, n_tx, active, Y, nullptr, 0, stream);
 }
 
 int wust_simulate(const double *c_mps, int ny, int nx, double dy_m, double dx_m, double dt_s, int n_time,

@@ -121,10 +121,12 @@ int ncg_project_launch(double *c, const double *d, double step, double max_updat
                        const uint8_t *mask, size_t n, double *part, cudaStream_t st);
 
 // ---- prepare.cu (DTFT of the RF preparation) --------------------------------
-// time_s, freq, K (nf x nt): device; rf [nt, n_rx, n_tx] float or double;
-// active [n_tx, n_rx] bytes; Y [n_tx, n_rx, nf]; *bad set on a nonfinite active sample.
+// time_s, freq: host; rf [nt, n_rx, n_tx] float or double, active [n_tx, n_rx]
+// bytes, workspace (dtft_workspace_bytes), Y [n_tx, n_rx, nf]: device;
+// **bad_out (in the workspace) is set on a nonfinite active sample.
+size_t dtft_workspace_bytes(int nt, int nf);
 void dtft_launch(const double *time_s, const double *freq, int nt, int nf, double dt, const void *rf, bool rf_double,
-                 int n_rx, int n_tx, const uint8_t *active, double2 *K, float2 *Y, int *bad, cudaStream_t st);
+                 int n_rx, int n_tx, const uint8_t *active, void *workspace, float2 *Y, int **bad_out, cudaStream_t st);
 
 // ---- nsfactor.cu (Newton-Schulz Schur inverses, TF32 tensor cores) ---------
 struct NsGeom {
