@@ -96,7 +96,8 @@ def dtft_device(time_s, frequencies_hz, pressure, active, stream=None):
     # the tables' room from torch's allocator: the library's own allocation maps and unmaps memory on every call.
     # The call has synchronized the stream when it returns, so the block may go back at once.
     need = lib.wust_dtft_workspace_bytes(t.size, f.size)
-    ws = torch.empty(need + 256, dtype=torch.uint8, device=dev)
+    with torch.cuda.stream(st):
+        ws = torch.empty(need + 256, dtype=torch.uint8, device=dev)
     at = -(-ws.data_ptr() // 256) * 256
     check(lib.wust_dtft_ws(t.ctypes.data_as(C.c_void_p), t.size, f.ctypes.data_as(C.c_void_p), f.size,
                            C.c_void_p(p.data_ptr()), int(is_double), n_rx, n_tx, C.c_void_p(act.data_ptr()),
