@@ -296,6 +296,17 @@ int wust_simulate(const double *c_mps, int ny, int nx, double dy_m, double dx_m,
                   const double *source, const int *tx_index, int n_tx, const int *rx_index, int n_rx, int pml_size,
                   double c_ref_mps, double rho0_kg_m3, int decimation, int tx_batch, float *rf, void *stream);
 
+/* wust_simulate for callers that keep device memory of their own: workspace is
+ * device memory of at least wust_simulate_workspace_bytes(...) bytes (0 where
+ * the call would not use it) on a 256-byte boundary, used until the call
+ * returns (NULL: the call allocates and frees it, as wust_simulate does). */
+size_t wust_simulate_workspace_bytes(int ny, int nx, int pml_size, int n_tx, int n_rx, int n_time, int decimation,
+                                     int tx_batch);
+int wust_simulate_ws(const double *c_mps, int ny, int nx, double dy_m, double dx_m, double dt_s, int n_time,
+                     const double *source, const int *tx_index, int n_tx, const int *rx_index, int n_rx, int pml_size,
+                     double c_ref_mps, double rho0_kg_m3, int decimation, int tx_batch, float *rf, void *workspace,
+                     size_t workspace_bytes, void *stream);
+
 /* Counters of the last solve/oracle call: correction solves of the last
  * refined solve, its final relative FP64 residual |b - Hx| / |b| and forward
  * error estimate (refined profiles; -1 otherwise), and the number of kernel

@@ -1169,9 +1169,23 @@ int wust_dtft(const double *time_s, int n_time, const double *frequencies_hz, in
     return wust_dtft_ws(time_s, n_time, frequencies_hz, n_f, rf, rf_is_double, n_rx, n_tx, active, Y, nullptr, 0, stream);
 }
 
+size_t wust_simulate_workspace_bytes(int ny, int nx, int pml_size, int n_tx, int n_rx, int n_time, int decimation,
+                                     int tx_batch) {
+    if (ny < 1 || nx < 1 || pml_size < 1 || n_tx < 1 || n_rx < 1 || n_time < 1 || decimation < 1) return 0;
+    return simulate_workspace_bytes(ny, nx, pml_size, n_tx, n_rx, n_time, decimation, tx_batch);
+}
+
 int wust_simulate(const double *c_mps, int ny, int nx, double dy_m, double dx_m, double dt_s, int n_time,
                   const double *source, const int *tx_index, int n_tx, const int *rx_index, int n_rx, int pml_size,
                   double c_ref_mps, double rho0_kg_m3, int decimation, int tx_batch, float *rf, void *stream) {
+    return wust_simulate_ws(c_mps, ny, nx, dy_m, dx_m, dt_s, n_time, source, tx_index, n_tx, rx_index, n_rx, pml_size,
+                            c_ref_mps, rho0_kg_m3, decimation, tx_batch, rf, nullptr, 0, stream);
+}
+
+int wust_simulate_ws(const double *c_mps, int ny, int nx, double dy_m, double dx_m, double dt_s, int n_time,
+                     const double *source, const int *tx_index, int n_tx, const int *rx_index, int n_rx, int pml_size,
+                     double c_ref_mps, double rho0_kg_m3, int decimation, int tx_batch, float *rf, void *workspace,
+                     size_t workspace_bytes, void *stream) {
     return guarded([&] {
         if (!c_mps || !source || !tx_index || !rx_index || !rf) fail(WUST_ERR_INVALID_INPUT, "simulate arguments missing");
         if (ny < 1 || nx < 1 || n_tx < 1 || n_rx < 1) fail(WUST_ERR_INVALID_INPUT, "Invalid medium");
@@ -1201,7 +1215,12 @@ int wust_simulate(const double *c_mps, int ny, int nx, double dy_m, double dx_m,
         }
         SimulateArgs a{c_mps, ny, nx, dy_m, dx_m, dt_s, n_time, source, tx_index, n_tx, rx_index, n_rx, pml_size,
                        c_ref_mps, rho0_kg_m3, decimation, tx_batch};
-        simulate_rf(a, rf, static_cast<cudaStream_t>(stream));
+        if (workspace) {
+            const size_t need = simulate_workspace_bytes(ny, nx, pml_size, n_tx, n_rx, n_time, decimation, tx_batch);
+            if (workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0)
+                fail(WUST_ERR_INVALID_INPUT, "simulate workspace of %zu bytes on 256 required", need);
+        }
+        simulate_rf(a, workspace, rf, static_cast<cudaStream_t>(stream));
     });
 }
 

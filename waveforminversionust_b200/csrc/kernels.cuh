@@ -249,6 +249,9 @@ struct SimulateArgs {
     int decimation;           // >= 1
     int tx_batch;             // transmitters per batch (0: all)
 };
-void simulate_rf(const SimulateArgs &a, float *rf, cudaStream_t st);
+// workspace: simulate_workspace_bytes of device memory (0: none is used), or
+// null to allocate it for the call.
+size_t simulate_workspace_bytes(int ny, int nx, int pml, int ntx, int nrx, int nt, int decimation, int tx_batch);
+void simulate_rf(const SimulateArgs &a, void *workspace, float *rf, cudaStream_t st);
 
 }  // namespace wust

@@ -101,10 +101,21 @@ def wust_simulate(model: dict, cfg: dict, stream=None) -> dict:
     batch = 0 if cfg["backend"] == "native-batch" else 1
     if "tx_batch" in cfg:
         batch = int(cfg["tx_batch"])
+    # the fields' room from torch's allocator: the library's own allocation maps and unmaps memory on every call.
+    # The call has synchronized the stream when it returns, so the block may go back at once.
+    need = lib.wust_simulate_workspace_bytes(ny, nx, pml, n_tx, n_rx, n_time, q, batch)
+    ws = None
+    if need:
+        with torch.cuda.stream(st):
+            try:
+                ws = torch.empty(need + 256, dtype=torch.uint8, device="cuda")
+            except torch.OutOfMemoryError:            # the library reports what it cannot allocate
+                pass
+    at = C.c_void_p(-(-ws.data_ptr() // 256) * 256) if ws is not None else None
     t0 = time.perf_counter()
-    check(lib.wust_simulate(cm.ctypes.data_as(C.c_void_p), ny, nx, dy, dx, dt, n_time, src.ctypes.data_as(C.c_void_p),
-                            ti.ctypes.data_as(C.c_void_p), n_tx, ri.ctypes.data_as(C.c_void_p), n_rx, pml, c_ref,
-                            rho0, q, batch, C.c_void_p(rf.data_ptr()), C.c_void_p(st.cuda_stream)))
+    check(lib.wust_simulate_ws(cm.ctypes.data_as(C.c_void_p), ny, nx, dy, dx, dt, n_time, src.ctypes.data_as(C.c_void_p),
+                               ti.ctypes.data_as(C.c_void_p), n_tx, ri.ctypes.data_as(C.c_void_p), n_rx, pml, c_ref,
+                               rho0, q, batch, C.c_void_p(rf.data_ptr()), at, need, C.c_void_p(st.cuda_stream)))
     generation = time.perf_counter() - t0
     pressure = rf.permute(2, 1, 0).cpu().numpy()      # [time, rx, tx]
     t_array = np.arange(n_time) * dt
