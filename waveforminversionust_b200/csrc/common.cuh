@@ -82,6 +82,17 @@ __device__ __forceinline__ unsigned long long global_timer_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+// Budget of a bounded wait.  The clock starts at the first question, which a
+// wait asks after some failed tries: reading the timer costs more than most
+// waits take (the end of a sweep step's products was seen 0.5 us late).
+struct WaitBudget {
+    unsigned long long t0 = 0;
+    __device__ __forceinline__ bool spent(unsigned long long timeout_ns) {
+        const unsigned long long t = global_timer_ns();
+        if (!t0) t0 = t;
+        return t - t0 > timeout_ns;
+    }
+};
 
 // ---------------------------------------------------------------------------
 // Coefficient views: the nine block arrays in the reference layout

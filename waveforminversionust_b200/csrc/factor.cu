@@ -77,13 +77,13 @@ __device__ __forceinline__ bool grid_barrier(unsigned *counter, int *err, unsign
         const unsigned target = epoch * nblocks;
         asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(counter), "r"(1u) : "memory");
         int ok = 1;
-        const unsigned long long t0 = global_timer_ns();
+        WaitBudget budget;
         for (unsigned spin = 0;; ++spin) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
             if ((int)(v - target) >= 0) break;
             if (*(volatile int *)err) { ok = 0; break; }
-            if ((spin & 31u) == 31u && global_timer_ns() - t0 > timeout_ns) {
+            if ((spin & 31u) == 31u && budget.spent(timeout_ns)) {
                 atomicCAS(err, 0, site);
                 ok = 0;
                 break;

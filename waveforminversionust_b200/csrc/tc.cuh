@@ -78,7 +78,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
 // Bounded parity wait: false when the budget ran out.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t phase, unsigned long long timeout_ns) {
     const uint32_t a = smem_u32(bar);
-    unsigned long long t0 = 0;
+    WaitBudget budget;
     for (uint32_t spin = 0;; ++spin) {
         uint32_t done;
         asm volatile(
@@ -87,11 +87,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t phase, unsigne
             : "r"(a), "r"(phase)
             : "memory");
         if (done) return true;
-        if ((spin & 63u) == 0) {
-            const unsigned long long t = global_timer_ns();
-            if (!t0) t0 = t;
-            else if (t - t0 > timeout_ns) return false;
-        }
+        if ((spin & 63u) == 63u && budget.spent(timeout_ns)) return false;
     }
 }
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
@@ -119,6 +115,9 @@ __device__ __forceinline__ void bulk_g2s_hint(void *dst, const void *src, uint32
         "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(pol)
         : "memory");
 }
+__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ uint64_t smem_desc(const void *p) {
     uint64_t d = 0;
     d |= (uint64_t)((smem_u32(p) >> 4) & 0x3FFF);                 // start address
@@ -127,6 +126,9 @@ __device__ __forceinline__ uint64_t smem_desc(const void *p) {
     d |= (uint64_t)1 << 46;                                       // descriptor version for sm_100
     return d;                                                     // base offset 0, no swizzle
 }
+// Another address (in units of 16 bytes, its field's overflow excluded) under
+// the same layout: the low word alone changes.
+__device__ __forceinline__ uint64_t desc_at(uint32_t low, uint64_t desc) { return (desc & 0xffffffff00000000ull) | low; }
 // Instruction descriptor: D fp32, A/B tf32 (kind::tf32) or bf16 (kind::f16), both K-major.
 template <bool TF32>
 __host__ __device__ constexpr uint32_t instr_desc(int m, int n) {

@@ -40,18 +40,18 @@ namespace wust {
 
 constexpr int kCkThreads = 512;
 constexpr int kCkWarps = kCkThreads / 32;
-constexpr int kCkStages = 4;
-constexpr int kCopyTid = 96;                                     // the ring's copy thread (warp 3, lane 0)
+constexpr int kCkMinStages = 4, kCkMaxStages = 10;
+constexpr int kCopyTid = 96, kCopyBTid = 128;                    // the ring's copy threads, of A and of B (lanes 0)
 constexpr int kCkMaxN = 256;                                     // sources per launch (MMA N)
 constexpr int kCkRowsPerChunk = 16;                              // complex rows per K chunk (TF32)
 constexpr int kCkRowsPerChunk16 = 32;                            // complex rows per K chunk (BF16)
 constexpr int kCkMaxChunks = 148;
 constexpr size_t kCkBSlot = (size_t)kCkMaxN * tc::kChunkBytes;   // 32 KB
-constexpr size_t kCkSmemRing = (size_t)kCkStages * (tc::kAChunk + kCkBSlot);
+constexpr size_t kCkSmemRing = (size_t)kCkMinStages * (tc::kAChunk + kCkBSlot);
 constexpr size_t kCkSmemHalo = 2 * kCkMaxN * sizeof(float2);
 constexpr size_t kCkSmemW = 3 * 64 * sizeof(float2);
 constexpr size_t kCkSmem = kCkSmemRing + kCkSmemHalo + kCkSmemW + 256;
-static_assert((size_t)kCkStages * kCkBSlot >= (size_t)kCkMaxN * 64 * sizeof(float2), "B stages hold the staged state");
+static_assert((size_t)kCkMinStages * tc::kChunkBytes >= 64 * sizeof(float2), "B stages hold the staged state");
 static_assert(kCkSmem <= 232448, "shared memory of one CTA");
 
 __host__ __device__ constexpr int ceil_div8(int x) { return (x + 7) / 8 * 8; }
@@ -135,29 +135,35 @@ struct ChunkParams {
     int ny, nx, n, mt, kc, N;
     int s0, s_end;            // global sources [s0, s_end) of this launch
     int half;                 // 0: forward substitution (steps 0 .. nx-2), 1: backward
+    int stages, per_stage;    // of the operand ring; K chunks per stage
     int pass, C;
     int bounds[kCkMaxChunks + 1];   // first step (within the half) of each chunk
     unsigned long long timeout_ns;
 };
+
+// Where the staged state holds row r of source s: pairs of rows, permuted
+// within eight so that a pair of 8 sources lies in 8 different bank groups.
+__device__ __forceinline__ int cs_at(int s, int r) { return s * 64 + (r ^ ((s & 7) << 1)); }
 
 // BF: BF16 operands (kind::f16 MMAs, 32 complex rows per K chunk) for the
 // correction solves of the refinement; TF32 otherwise.
 template <bool ADJ, bool BF>
 __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_constant__ ChunkParams p) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t *sA = smem;                                          // [stage] 16 KB
-    uint8_t *sB = smem + (size_t)kCkStages * tc::kAChunk;        // [stage] 32 KB
+    const int stages = p.stages, G = p.per_stage, kg = (p.kc + G - 1) / G;
+    uint8_t *sA = smem;                                          // [stage] G chunks of 16 KB
+    uint8_t *sB = smem + (size_t)stages * G * tc::kAChunk;       // [stage] G chunks of N x 128 bytes
     // Between a step's MMAs and the next step's B copies the B stages hold the
-    // state of this CTA's 64 rows: cs[s * 64 + row] (complex).
+    // state of this CTA's 64 rows: cs[cs_at(s, row)] (complex).
     float2 *cs = reinterpret_cast<float2 *>(sB);
     float2 *halo = reinterpret_cast<float2 *>(smem + kCkSmemRing);  // [2][kCkMaxN]: rows 64t-1 and 64t+64
     float2 *wts = halo + 2 * kCkMaxN;                                // [3][64] stencil weights of own rows
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + kCkSmemRing + kCkSmemHalo + kCkSmemW);
-    uint64_t *empty = full + kCkStages;
-    uint64_t *done = empty + kCkStages;
+    uint64_t *empty = full + kCkMaxStages;
+    uint64_t *done = empty + kCkMaxStages;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 1);
     int *s_ok = reinterpret_cast<int *>(tmem_slot + 1);
-    uint32_t *s_ring = reinterpret_cast<uint32_t *>(s_ok + 1);   // [0] A, [1] B copies issued, [2] full waits done
+    uint32_t *s_ring = reinterpret_cast<uint32_t *>(s_ok + 1);   // [0] A, [1] B copies issued
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = blockIdx.x / p.mt, t = blockIdx.x % p.mt;
@@ -211,7 +217,7 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
     // staged state at complex interior row yp (row0 - 1 .. row0 + 64)
     auto cs_get = [&](int yp, int s) -> float2 {
         const int l = yp - row0;
-        if (l >= 0 && l < 64) return cs[s * 64 + l];
+        if (l >= 0 && l < 64) return cs[cs_at(s, l)];
         if (l == -1) return halo[s];
         if (l == 64) return halo[kCkMaxN + s];
         return f2(0.f, 0.f);
@@ -229,7 +235,7 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int it = it0 + q * kCkThreads;
-                if (it < 64 * N) cs[(it >> 6) * 64 + (it & 63)] = v[q];
+                if (it < 64 * N) cs[cs_at(it >> 6, it & 63)] = v[q];
             }
         }
         for (int it = tid; it < 2 * N; it += kCkThreads) {
@@ -271,8 +277,7 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
     //   P_TURN     the turn of the H^H solve: u(:, nx-1) = SRC_{nx-1} -
     //              U_{nx-2}^H c on every row, no B.
     // Exact H^H forward steps also write B into u(:, j-1) (stencil mode:
-    // with its border rows).  Warp w handles sources w, w+8, ...; lane r the
-    // rows 2r, 2r+1 (neighbour rows by shuffles).
+    // with its border rows).
     auto produce = [&](int k, int mode, float *out, bool wts_ready) {
         bool fwd1 = true;
         int j1 = nx;
@@ -298,97 +303,145 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
                 p.u[plane * gs + (size_t)ny * (j1 - 1) + y] =
                     csub(step_base<ADJ>(p.src, p.u, ny, nx, fwd1, j1, y, gs), acc);
             }
-            __syncthreads();                               // the packing below overwrites the staged state
+            __syncthreads();                               // below, the results replace the staged state
         }
-        const int yp0 = row0 + 2 * lane, y0 = yp0 + 1;
-        const bool v0 = yp0 < n, v1 = yp0 + 1 < n;
-        const float2 wc0 = wts[2 * lane], wm0 = wts[64 + 2 * lane], wp0 = wts[128 + 2 * lane];
-        const float2 wc1 = wts[2 * lane + 1], wm1 = wts[64 + 2 * lane + 1], wp1 = wts[128 + 2 * lane + 1];
-        const int q_own = min(4, kc - row0 / kCkRowsPerChunk);    // packed chunks of this CTA's rows
-        // Warp: groups of 8 consecutive sources.  The packed chunks take the
-        // 8 sources of one row pair as one 128-byte row, so the warp writes
-        // its results over its own (already consumed) 4 KB of staged state in
-        // that order (XOR-swizzled against bank conflicts) and copies them out
-        // as contiguous 512-byte stores.
-        for (int grp = warp; grp < N / 8; grp += kCkWarps) {
-            float4 bq[8];
+        // base of the step (step_base), what does not depend on the source taken out of the loop
+        const float2 *bcol = nullptr;
+        bool point = false, scatter = false;
+        int col_at = 0;
+        if (has_base && fwd1 && (!ADJ || j1 >= 2)) {
+            const int jb = ADJ ? j1 - 1 : j1;
+            col_at = row0 + 1 + ny * jb;
+            if (p.src.mode == SRC_DENSE) bcol = p.src.dense + (size_t)ny * jb;
+            point = p.src.mode == SRC_POINT;
+            scatter = p.src.mode == SRC_SCATTER;
+        } else if (has_base && ADJ && !fwd1) {
+            bcol = p.u + (size_t)ny * j1;
+        }
+        const bool fields = bcol || wu || out;      // columns of fields are read or written
+        // Where columns of fields are involved, a first pass forms B in place of
+        // the staged state, rows in lanes, so that each access to a field is a
+        // run of 32 rows.  The second packs it (and, without fields, forms it):
+        // a lane takes one 16-byte unit of one source, a warp 4 units of 8
+        // sources, 512 bytes of a packed chunk in a row, straight from registers.
+        // Loops stay rolled: a step runs all of its code once, and straight-line
+        // code for 8 sources was bound by instruction fetch (produce at 16
+        // sources 2.5 us, here 0.8; at 128 4.5 against 2.7 without fields).
+        // Per step of 256 sources 8.6 -> 9.0 us with fields, 192 without 5.2 -> 4.5.
+        constexpr int RPC = BF ? kCkRowsPerChunk16 : kCkRowsPerChunk;
+        constexpr int RPU = RPC / 8, NI = 16 / RPU;                   // rows of a 16-byte unit; items of 8 sources
+        if (fields) {
+            const int yl = row0 + lane + 1;                           // rows of this lane: yl and yl + 32
+            int at[2] = {col_at + lane, col_at + lane + 32};
+            if (scatter)
+                for (int h = 0; h < 2; ++h) at[h] = yl + 32 * h <= n ? p.src.at[at[h]] : -1;
+            float2 wc[2], wm[2], wp[2];
 #pragma unroll
-            for (int h4 = 0; h4 < 2; ++h4) {
-                float2 base[4][2];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int gs = p.s0 + so + 8 * grp + 4 * h4 + q;
-                    base[q][0] = base[q][1] = f2(0.f, 0.f);
-                    if (has_base && gs < p.s_end) {
-                        if (v0) base[q][0] = step_base<ADJ>(p.src, p.u, ny, nx, fwd1, j1, y0, gs);
-                        if (v1) base[q][1] = step_base<ADJ>(p.src, p.u, ny, nx, fwd1, j1, y0 + 1, gs);
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const int s = 8 * grp + 4 * h4 + q, gs = p.s0 + so + s;
-                    const float4 cv = *reinterpret_cast<const float4 *>(cs + s * 64 + 2 * lane);
-                    const float2 c0 = f2(cv.x, cv.y), c1 = f2(cv.z, cv.w);
-                    float2 cm = f2(__shfl_up_sync(0xffffffffu, c1.x, 1), __shfl_up_sync(0xffffffffu, c1.y, 1));
-                    float2 cp = f2(__shfl_down_sync(0xffffffffu, c0.x, 1), __shfl_down_sync(0xffffffffu, c0.y, 1));
-                    if (lane == 0) cm = halo[s];
-                    if (lane == 31) cp = halo[kCkMaxN + s];
-                    float2 b0 = f2(0.f, 0.f), b1 = b0;
-                    if (gs < p.s_end) {
-                        if (v0) {
-                            float2 acc = cmul(wc0, c0);
-                            cfma(acc, wm0, cm);
-                            cfma(acc, wp0, c1);
-                            b0 = csub(base[q][0], acc);
-                            if (wu) p.u[plane * gs + (size_t)ny * (j1 - 1) + y0] = b0;
-                        }
-                        if (v1) {
-                            float2 acc = cmul(wc1, c1);
-                            cfma(acc, wm1, c0);
-                            cfma(acc, wp1, cp);
-                            b1 = csub(base[q][1], acc);
-                            if (wu) p.u[plane * gs + (size_t)ny * (j1 - 1) + y0 + 1] = b1;
-                        }
-                        if (out) {
-                            float *re = out + (size_t)(so + s) * ny, *im = out + (size_t)(kCkMaxN + so + s) * ny;
-                            if (v0) { __stcg(re + y0, b0.x); __stcg(im + y0, b0.y); }
-                            if (v1) { __stcg(re + y0 + 1, b1.x); __stcg(im + y0 + 1, b1.y); }
-                        }
-                    }
-                    if (BF) {
-                        // rows yp0, yp0 + 1 of chunk yp0 / 32: four bf16 values (8 bytes)
-                        if (pack && yp0 < kCkRowsPerChunk16 * kc) {
-                            const int Q = yp0 / kCkRowsPerChunk16, ke = 2 * (yp0 % kCkRowsPerChunk16);
-                            const uint32_t lo = (uint32_t)tc::to_bf16_bits(b0.x) | ((uint32_t)tc::to_bf16_bits(b0.y) << 16);
-                            const uint32_t hi = (uint32_t)tc::to_bf16_bits(b1.x) | ((uint32_t)tc::to_bf16_bits(b1.y) << 16);
-                            *reinterpret_cast<uint2 *>(bg + (size_t)Q * bbytes + tc::chunk_off16(s, ke)) = make_uint2(lo, hi);
-                        }
-                    } else {
-                        bq[4 * h4 + q] = make_float4(to_tf32(b0.x), to_tf32(b0.y), to_tf32(b1.x), to_tf32(b1.y));
-                    }
-                }
+            for (int h = 0; h < 2; ++h) {
+                wc[h] = wts[lane + 32 * h];
+                wm[h] = wts[64 + lane + 32 * h];
+                wp[h] = wts[128 + lane + 32 * h];
             }
-            if (pack && !BF) {
-                float4 *reg = reinterpret_cast<float4 *>(cs + (size_t)grp * 8 * 64);   // 256 float4
-                __syncwarp();
+#pragma unroll 1
+            for (int s0 = 4 * warp; s0 < N; s0 += 4 * kCkWarps) {
+                float2 v[4][2];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) reg[lane * 8 + (q ^ (lane & 7))] = bq[q];
-                __syncwarp();
-                for (int Q = 0; Q < q_own; ++Q) {
+                for (int q = 0; q < 4; ++q) {
+                    const int gs = p.s0 + so + s0 + q;
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        const int idx = lane + 32 * h, kg = idx >> 3;
-                        const float4 v = reg[(Q * 8 + kg) * 8 + ((idx & 7) ^ kg)];
-                        *reinterpret_cast<float4 *>(bg + (size_t)(row0 / kCkRowsPerChunk + Q) * bbytes +
-                                                    (size_t)grp * 1024 + (size_t)idx * 16) = v;
+                        v[q][h] = f2(0.f, 0.f);
+                        if (gs >= p.s_end) continue;
+                        if (bcol) {
+                            if (yl + 32 * h <= n) v[q][h] = __ldcg(bcol + plane * gs + yl + 32 * h);
+                        } else if (point) {
+                            v[q][h].x = p.src.lin[gs] == at[h] ? 1.f : 0.f;
+                        } else if (scatter && at[h] >= 0) {
+                            v[q][h] = p.src.vals[at[h] + (size_t)p.src.n_slots * gs];
+                        }
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int s = s0 + q, gs = p.s0 + so + s;
+                    float2 c[2][3];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int r = lane + 32 * h;
+                        c[h][0] = r == 0 ? halo[s] : cs[cs_at(s, r - 1)];
+                        c[h][1] = cs[cs_at(s, r)];
+                        c[h][2] = r == 63 ? halo[kCkMaxN + s] : cs[cs_at(s, r + 1)];
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float2 acc = cmul(wc[h], c[h][1]);
+                        cfma(acc, wm[h], c[h][0]);
+                        cfma(acc, wp[h], c[h][2]);
+                        const bool on = gs < p.s_end && yl + 32 * h <= n;
+                        const float2 b = on ? csub(v[q][h], acc) : f2(0.f, 0.f);
+                        if (on && wu) p.u[plane * gs + (size_t)ny * (j1 - 1) + yl + 32 * h] = b;
+                        if (on && out) {
+                            __stcg(out + (size_t)(so + s) * ny + yl + 32 * h, b.x);
+                            __stcg(out + (size_t)(kCkMaxN + so + s) * ny + yl + 32 * h, b.y);
+                        }
+                        cs[cs_at(s, lane + 32 * h)] = b;
                     }
                 }
             }
+            if (!pack) return;
+            __syncthreads();
+        }
+#pragma unroll 1
+        for (int it = warp; it < N / 8 * NI; it += kCkWarps) {
+            const int unit = (it % NI) * 4 + (lane >> 3), r = unit * RPU, s = it / NI * 8 + (lane & 7);
+            const int gs = p.s0 + so + s;
+            float2 v[RPU], c[RPU + 2];
+#pragma unroll
+            for (int h = 0; h < RPU; h += 2) {
+                const float4 c2 = *reinterpret_cast<const float4 *>(cs + cs_at(s, r + h));
+                c[h + 1] = f2(c2.x, c2.y);
+                c[h + 2] = f2(c2.z, c2.w);
+            }
+            if (fields) {
+#pragma unroll
+                for (int h = 0; h < RPU; ++h) v[h] = c[h + 1];
+            } else {
+                c[0] = r == 0 ? halo[s] : cs[cs_at(s, r - 1)];
+                c[RPU + 1] = r + RPU == 64 ? halo[kCkMaxN + s] : cs[cs_at(s, r + RPU)];
+                const int src_row = point && gs < p.s_end ? p.src.lin[gs] - col_at : -1;
+#pragma unroll
+                for (int h = 0; h < RPU; ++h) {
+                    float2 acc = cmul(wts[r + h], c[h + 1]), base = f2(0.f, 0.f);
+                    cfma(acc, wts[64 + r + h], c[h]);
+                    cfma(acc, wts[128 + r + h], c[h + 2]);
+                    const bool on = gs < p.s_end && row0 + r + h < n;
+                    if (src_row == r + h) base.x = 1.f;
+                    if (scatter && on) {
+                        const int k1 = p.src.at[col_at + r + h];
+                        if (k1 >= 0) base = p.src.vals[k1 + (size_t)p.src.n_slots * gs];
+                    }
+                    v[h] = on ? csub(base, acc) : f2(0.f, 0.f);
+                }
+            }
+            const int at = row0 / RPU + unit;                         // unit of the group's B
+            if (at >= 8 * kc) continue;
+            float4 q;
+            if constexpr (BF) {
+                uint32_t w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    w[i] = (uint32_t)tc::to_bf16_bits(v[i].x) | ((uint32_t)tc::to_bf16_bits(v[i].y) << 16);
+                q = make_float4(__uint_as_float(w[0]), __uint_as_float(w[1]), __uint_as_float(w[2]), __uint_as_float(w[3]));
+            } else {
+                q = make_float4(to_tf32(v[0].x), to_tf32(v[0].y), to_tf32(v[1].x), to_tf32(v[1].y));
+            }
+            *reinterpret_cast<float4 *>(bg + (size_t)(at >> 3) * bbytes + (size_t)(s >> 3) * 1024 + (at & 7) * 128 + (s & 7) * 16) = q;
         }
     };
 
     if (tid == 0) {
-        for (int q = 0; q < kCkStages; ++q) {
+        for (int q = 0; q < stages; ++q) {
             tc::mbar_init(&full[q], 2);       // A copy + B copy
             tc::mbar_init(&empty[q], 1);      // MMAs of the stage retired
         }
@@ -416,13 +469,13 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
             float v[32];
             tc::tmem_ld32(tl + (uint32_t)(c0 + cb), v);
 #pragma unroll
-            for (int q = 0; q < 32; ++q) csf[((size_t)(c0 + cb + q) * 64 + row) * 2 + part] = row_ok ? v[q] : 0.f;
+            for (int q = 0; q < 32; ++q) csf[cs_at(c0 + cb + q, row) * 2 + part] = row_ok ? v[q] : 0.f;
         }
         for (; cb < hc && c0 + cb < N; cb += 8) {
             float v[8];
             tc::tmem_ld8(tl + (uint32_t)(c0 + cb), v);
 #pragma unroll
-            for (int q = 0; q < 8; ++q) csf[((size_t)(c0 + cb + q) * 64 + row) * 2 + part] = row_ok ? v[q] : 0.f;
+            for (int q = 0; q < 8; ++q) csf[cs_at(c0 + cb + q, row) * 2 + part] = row_ok ? v[q] : 0.f;
         }
     };
     // The state after step k: subtracting steps take old - value; write the
@@ -435,8 +488,8 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
         const bool wu = kind == K_EXACT && (!ADJ || !fwd);
         const float *oldp = kind == K_BOUND ? (ADJ ? p.sb : p.zst) + (size_t)(t0 + k) * sfl : nullptr;
         const bool old_u = sub && kind != K_BOUND && kind != K_PROP;
-        const int yp0 = row0 + 2 * lane, y0 = yp0 + 1;
-        const bool v0 = yp0 < n, v1 = yp0 + 1 < n;
+        const int y0 = row0 + lane + 1, y1 = y0 + 32;
+        const bool v0 = y0 <= n, v1 = y1 <= n;
         __syncthreads();
         for (int sb0 = warp; sb0 < N; sb0 += 4 * kCkWarps) {
             float2 o[4][2];
@@ -448,11 +501,11 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
                     if (old_u) {
                         const float2 *uc = p.u + plane * gs + (size_t)ny * j;
                         if (v0) o[q][0] = __ldcs(uc + y0);
-                        if (v1) o[q][1] = __ldcs(uc + y0 + 1);
+                        if (v1) o[q][1] = __ldcs(uc + y1);
                     } else if (kind == K_BOUND) {
                         const float *ore = oldp + (size_t)(so + s) * ny, *oim = oldp + (size_t)(kCkMaxN + so + s) * ny;
                         if (v0) o[q][0] = f2(__ldcg(ore + y0), __ldcg(oim + y0));
-                        if (v1) o[q][1] = f2(__ldcg(ore + y0 + 1), __ldcg(oim + y0 + 1));
+                        if (v1) o[q][1] = f2(__ldcg(ore + y1), __ldcg(oim + y1));
                     }
                 }
             }
@@ -460,28 +513,33 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
             for (int q = 0; q < 4; ++q) {
                 const int s = sb0 + kCkWarps * q, gs = p.s0 + so + s;
                 if (s >= N) break;                                   // warp-uniform
-                float4 *cp4 = reinterpret_cast<float4 *>(cs + s * 64 + 2 * lane);
-                float4 cv = *cp4;
+                float2 *e0 = cs + cs_at(s, lane), *e1 = cs + cs_at(s, lane + 32);
+                float2 c0 = *e0, c1 = *e1;
                 if (sub) {
-                    cv = make_float4(o[q][0].x - cv.x, o[q][0].y - cv.y, o[q][1].x - cv.z, o[q][1].y - cv.w);
-                    if (!v0) { cv.x = 0.f; cv.y = 0.f; }
-                    if (!v1) { cv.z = 0.f; cv.w = 0.f; }
-                    *cp4 = cv;
+                    c0 = v0 ? csub(o[q][0], c0) : f2(0.f, 0.f);
+                    c1 = v1 ? csub(o[q][1], c1) : f2(0.f, 0.f);
+                    *e0 = c0;
+                    *e1 = c1;
                 }
                 if (gs >= p.s_end) continue;
                 if (wu) {                 // u streams through L2 (evict first), as the old column it replaces
                     float2 *uc = p.u + plane * gs + (size_t)ny * j;
-                    if (v0) __stcs(uc + y0, f2(cv.x, cv.y));
-                    if (v1) __stcs(uc + y0 + 1, f2(cv.z, cv.w));
+                    if (v0) __stcs(uc + y0, c0);
+                    if (v1) __stcs(uc + y1, c1);
                 }
-                if (lane == 0) __stcg(my_edges + s, f2(cv.x, cv.y));
-                if (lane == 31 && v1) __stcg(my_edges + kCkMaxN + s, f2(cv.z, cv.w));
                 if (last) {
                     float *re = curp + (size_t)(so + s) * ny, *im = curp + (size_t)(kCkMaxN + so + s) * ny;
-                    if (v0) { __stcg(re + y0, cv.x); __stcg(im + y0, cv.y); }
-                    if (v1) { __stcg(re + y0 + 1, cv.z); __stcg(im + y0 + 1, cv.w); }
+                    if (v0) { __stcg(re + y0, c0.x); __stcg(im + y0, c0.y); }
+                    if (v1) { __stcg(re + y1, c1.x); __stcg(im + y1, c1.y); }
                 }
             }
+        }
+        // edge rows of the warp's sources
+        __syncwarp();
+        for (int it = lane; it < 2 * kCkMaxN / kCkWarps; it += 32) {
+            const int s = warp + kCkWarps * (it >> 1), e = it & 1;
+            if (s < N && p.s0 + so + s < p.s_end && (e == 0 || row0 + 63 < n))
+                __stcg(my_edges + e * kCkMaxN + s, cs[cs_at(s, 63 * e)]);
         }
         if (kind == K_EXACT && ADJ && !fwd && t == 0) {
             // H^H backward: border rows of u(:, j) are zero
@@ -526,53 +584,68 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
     };
 
     // ---- bulk-copy ring; chunk ci = k * kc + q of step k --------------------
-    // Two threads drive it: the copy thread (kCopyTid) refills each stage as
-    // soon as the MMAs that read it have completed, and thread 0 issues each
-    // chunk's MMAs as soon as its copies have landed, so neither waits on
-    // the other's latency.  A chunk's stage is slot ci % kCkStages, used for
-    // the (ci / kCkStages)-th time.
-    uint32_t a_next = 0, b_next = 0, full_waited = 0;
+    // Three threads drive it: the copy threads (kCopyTid for A, kCopyBTid for
+    // B) refill each stage as soon as the MMAs that read it have completed,
+    // and thread 0 issues each chunk's MMAs as soon as its copies have landed,
+    // so none waits on another's latency.  Chunk ci's stage is slot ci %
+    // stages, used for the (ci / stages)-th time; each thread counts its slots
+    // and phases along.  Up to N = 128 the ring is bound by what these threads
+    // do per stage rather than by bytes or products: with divisions by kc and
+    // the ring's length per chunk, and the timer read in each wait, a step's
+    // ring took 13.3 us at 552^2 (TF32 and BF16 steps of 256 sources averaged),
+    // 9.9 at 437 x 401 and 6.6 at 288^2 (128 sources), 12.0, 9.1 and 6.0 in the
+    // boundary chain; now 9.7, 5.9, 3.9 and 7.5, 5.3, 3.6.  An L2 prefetch of the
+    // next step's pages while the MMAs' results are finished: TF32 steps 4 %
+    // slower.
+    int c_slot = 0, c_q = 0, a_k = 0;                            // a copy thread's next chunk; thread 0: the next MMAs
+    uint32_t c_next = 0, c_phase = 0;
+    const uint8_t *a_src = nullptr;
     // the page stream passes through L2 once; the packed B is read by every
     // CTA of the group and should stay
-    const uint64_t a_policy = tc::policy_evict_first();
-    const uint64_t b_policy = tc::policy_evict_last();
-    // copy thread: the A chunk a_next into its stage, once the MMAs of the
-    // chunk that used the stage before have completed
-    auto issue_a = [&]() -> bool {
-        const uint32_t c = a_next;
-        const int ks = (int)(c / kc), q = (int)(c % kc), slot = (int)(c % kCkStages);
-        if (c >= (uint32_t)kCkStages && !tc::mbar_wait(&empty[slot], ((c / kCkStages) - 1) & 1u, p.timeout_ns))
-            return false;
-        tc::mbar_expect_tx(&full[slot], tc::kAChunk);
-        tc::bulk_g2s_hint(sA + (size_t)slot * tc::kAChunk, apage(ks) + ((size_t)t * kc + q) * tc::kAChunk, tc::kAChunk,
-                          &full[slot], a_policy);
-        ++a_next;
-        return true;
+    const uint64_t policy = tid == kCopyTid && kind != K_BOUND ? tc::policy_evict_first() : tc::policy_evict_last();
+    auto advance = [&]() {
+        ++c_next;
+        if (++c_slot == stages) { c_slot = 0; c_phase ^= 1u; }
     };
-    // copy thread, step k: every B chunk of the step (each after its A
-    // chunk), then the next step's first A chunks as the stages free up
-    auto copies = [&](int k) {
-        bool good = true;
-        const uint32_t end = (uint32_t)(k + 1) * (uint32_t)kc;
-        while (good && b_next < end) {
-            if (a_next <= b_next && !(good = issue_a())) break;
-            const int q = (int)(b_next % kc), slot = (int)(b_next % kCkStages);
-            tc::mbar_expect_tx(&full[slot], (uint32_t)bbytes);
-            tc::bulk_g2s_hint(sB + (size_t)slot * kCkBSlot, bg + (size_t)q * bbytes, (uint32_t)bbytes, &full[slot],
-                              b_policy);
-            ++b_next;
+    // the next chunk of a copy thread may go into its stage
+    auto stage_free = [&]() { return c_next < (uint32_t)stages || tc::mbar_wait(&empty[c_slot], c_phase ^ 1u, p.timeout_ns); };
+    // A: stages up to `end`
+    auto copies_a = [&](uint32_t end) {
+        while (c_next < end) {
+            if (!stage_free()) {
+                atomicCAS(p.err, 0, SITE_COPY);
+                return;
+            }
+            if (c_q == 0) a_src = apage(a_k++) + (size_t)t * kc * tc::kAChunk;
+            const uint32_t bytes = (uint32_t)min(G, kc - c_q) * (uint32_t)tc::kAChunk;
+            tc::mbar_expect_tx(&full[c_slot], bytes);
+            tc::bulk_g2s_hint(sA + c_slot * (G * (uint32_t)tc::kAChunk), a_src, bytes, &full[c_slot], policy);
+            a_src += bytes;
+            c_q += G;
+            if (c_q >= kc) c_q = 0;
+            advance();
         }
-        const uint32_t a_end = min((uint32_t)min(k + 2, nsteps) * (uint32_t)kc, end + (uint32_t)kCkStages);
-        while (good && a_next < a_end) good = issue_a();
-        if (!good) atomicCAS(p.err, 0, SITE_COPY);
+    };
+    // B: every stage of a step
+    auto copies_b = [&]() {
+        const uint8_t *src = bg;
+        for (int q = 0; q < kc; q += G) {
+            if (!stage_free()) {
+                atomicCAS(p.err, 0, SITE_COPY);
+                return;
+            }
+            const uint32_t bytes = (uint32_t)min(G, kc - q) * (uint32_t)bbytes;
+            tc::mbar_expect_tx(&full[c_slot], bytes);
+            tc::bulk_g2s_hint(sB + c_slot * (G * (uint32_t)bbytes), src, bytes, &full[c_slot], policy);
+            src += bytes;
+            advance();
+        }
     };
 
     unsigned epoch = 0;
     bool ok = nsteps > 0;
     if (ok) {
-        if (tid == kCopyTid)                                // the first A chunks of step 0
-            while (a_next < (uint32_t)min(kCkStages, kc) && issue_a()) {
-            }
+        if (tid == kCopyTid) copies_a((uint32_t)min(stages, kg));      // the first A chunks of step 0
         int in0 = IN_ZERO, mode0 = P_STENCIL;
         const float *pl0 = nullptr;
         if (kind == K_EXACT && chunk > 0) {
@@ -598,6 +671,7 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
     float *cur = kind == K_BOUND ? nullptr : p.zst + (size_t)chunk * sfl;
     constexpr int kMmaPerChunk = tc::kChunkBytes / 32;
     const uint32_t idesc = tc::instr_desc<!BF>(tc::kTileRows, N);
+    const uint64_t desc_a = tc::smem_desc(sA), desc_b = tc::smem_desc(sB);
 
 #ifdef WUST_CHUNK_PROFILE
     long long prof_t = clock64();
@@ -605,26 +679,36 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
 #endif
     for (int k = 0; k < nsteps && ok; ++k) {
         CPROF(6);
-        if (tid == kCopyTid) copies(k);
+        // this step's chunks, and the next one's first A chunks as stages free up
+        if (tid == kCopyTid)
+            copies_a(min((uint32_t)min(k + 2, nsteps) * (uint32_t)kg, (uint32_t)(k + 1) * (uint32_t)kg + (uint32_t)stages));
+        if (tid == kCopyBTid) copies_b();
         if (tid == 0) {
             bool good = true;
-            for (int q = 0; q < kc; ++q) {
-                const uint32_t ci = (uint32_t)k * kc + q;
-                const int slot = (int)(ci % kCkStages);
-                if (!tc::mbar_wait(&full[slot], (ci / kCkStages) & 1u, p.timeout_ns)) { good = false; break; }
-                full_waited = ci + 1;
-                tc::fence_after();
+            auto chunk_mmas = [&](uint32_t da, uint32_t db, bool first) {
 #pragma unroll
                 for (int kk = 0; kk < kMmaPerChunk; ++kk)
-                    tc::mma<!BF>(tmem, tc::smem_desc(sA + (size_t)slot * tc::kAChunk + kk * 256),
-                                  tc::smem_desc(sB + (size_t)slot * kCkBSlot + kk * 256), idesc,
-                                  (q > 0 || kk > 0) ? 1u : 0u);
-                tc::commit(&empty[slot]);
+                    tc::mma<!BF>(tmem, tc::desc_at(da + kk * 16, desc_a), tc::desc_at(db + kk * 16, desc_b), idesc,
+                                 first && kk == 0 ? 0u : 1u);
+            };
+            const uint32_t step_a = G * (uint32_t)(tc::kAChunk / 16), step_b = G * (uint32_t)(bbytes / 16);
+            uint32_t da = (uint32_t)desc_a + c_slot * step_a, db = (uint32_t)desc_b + c_slot * step_b;
+            for (int q = 0; q < kc; q += G) {
+                if (!tc::mbar_wait(&full[c_slot], c_phase, p.timeout_ns)) { good = false; break; }
+                tc::fence_after();
+                chunk_mmas(da, db, q == 0);
+                if (G > 1)
+                    for (int i = 1; i < min(G, kc - q); ++i)
+                        chunk_mmas(da + i * (uint32_t)(tc::kAChunk / 16), db + i * (uint32_t)(bbytes / 16), false);
+                tc::commit(&empty[c_slot]);
+                advance();
+                da = c_slot ? da + step_a : (uint32_t)desc_a;
+                db = c_slot ? db + step_b : (uint32_t)desc_b;
             }
             tc::commit(done);
             if (!good) atomicCAS(p.err, 0, SITE_COPY);
         }
-        if (warp >= 1 && tid != kCopyTid) prefetch_cols(k);
+        if (warp >= 1 && tid != kCopyTid && tid != kCopyBTid) prefetch_cols(k);
         if (warp == 1 || warp == 2) {
             const bool next_b = k + 1 < nsteps || (ADJ && p.pass == CK_FIRST && chunk + 1 < p.C);
             if (next_b) {
@@ -675,19 +759,17 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
         }
     }
 
-    // copies issued but never waited for (a failure): stand in for the B
-    // copies that will not come, then let them land (bounded)
-    if (tid == kCopyTid) {
-        s_ring[0] = a_next;
-        s_ring[1] = b_next;
-    }
-    if (tid == 0) s_ring[2] = full_waited;
+    // copies issued but never waited for (a failure, in which one of the two
+    // may have stopped short): stand in for those that will not come, then let
+    // the others land (bounded)
+    if (tid == kCopyTid) s_ring[0] = c_next;
+    if (tid == kCopyBTid) s_ring[1] = c_next;
     __syncthreads();
     if (tid == 0) {
-        for (uint32_t ci = s_ring[2]; ci < s_ring[0]; ++ci) {
-            const int slot = (int)(ci % kCkStages);
-            if (ci >= s_ring[1]) tc::mbar_arrive(&full[slot]);
-            tc::mbar_wait(&full[slot], (ci / kCkStages) & 1u, p.timeout_ns);
+        for (; c_next < max(s_ring[0], s_ring[1]); advance()) {
+            for (int h = 0; h < 2; ++h)
+                if (c_next >= s_ring[h]) tc::mbar_arrive(&full[c_slot]);
+            tc::mbar_wait(&full[c_slot], c_phase, p.timeout_ns);
         }
     }
     tc::fence_before();
@@ -924,6 +1006,15 @@ static void set_bounds(ChunkParams &p, int C, bool adjoint, int half) {
 static void ck_launch(ChunkParams &p, bool adjoint, bool bf16, int pass, int groups, cudaStream_t st) {
     if (groups <= 0) return;
     p.pass = pass;
+    // As many stages as the shared memory holds, and K chunks per stage so that
+    // a stage's products take about as long as its share of the waits, commits
+    // and copies: a 16-row chunk of 256 sources is 512 cycles of MMAs, of 128
+    // sources 256, of 16 (the boundary chain) 192.  Measured with 4 / 2 / 1
+    // chunks per stage against 1: 288^2 Hessian product 26.9 against 28.5 ms,
+    // 437 x 401 solve 16.6 against 17.9; two at N = 256 (two stages left in the
+    // ring): 552^2 gradient 70.5 against 68.3.
+    p.per_stage = p.N <= 64 ? 4 : p.N <= 128 ? 2 : 1;
+    p.stages = std::min<int>(kCkMaxStages, (int)(kCkSmemRing / (p.per_stage * (tc::kAChunk + (size_t)p.N * tc::kChunkBytes))));
     WUST_CUDA(cudaMemsetAsync(p.group_ctr, 0, sizeof(unsigned) * groups, st));
     void *args[] = {&p};
     const dim3 grid(groups * p.mt), block(kCkThreads);

@@ -24,14 +24,14 @@ __device__ __forceinline__ bool counter_sync(unsigned *ctr, unsigned target, int
         asm volatile("fence.proxy.async.global;" ::: "memory");
         asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(ctr), "r"(1u) : "memory");
         int ok = 1;
-        const unsigned long long t0 = global_timer_ns();
+        WaitBudget budget;
         for (unsigned spin = 0;; ++spin) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
             if ((int)(v - target) >= 0) break;
             if ((spin & 15u) == 15u) {
                 if (*(volatile int *)err) { ok = 0; break; }
-                if (global_timer_ns() - t0 > timeout_ns) {
+                if (budget.spent(timeout_ns)) {
                     atomicCAS(err, 0, site);
                     ok = 0;
                     break;
