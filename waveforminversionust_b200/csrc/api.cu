@@ -105,7 +105,7 @@ struct wust_solver {
     bool fft_ready = false;
     cufftHandle fft_fwd = 0, fft_inv = 0;
     double2 *spec = nullptr;
-    double *ncg_part = nullptr;
+    NcgReduce ncg{};                 // one block of device memory
     double f = 0, sgn = -1, a0 = 0, L = 0, vmin = 0, vmax = 0;
     int ldr9 = 0;
     double dt = 0, cr = 0;
@@ -231,7 +231,7 @@ static void free_solver(wust_solver *s) {
         cufftDestroy(s->fft_inv);
     }
     dfree(s->spec);
-    dfree(s->ncg_part);
+    dfree(s->ncg.part);
     for (int i = 0; i < 9; ++i) { dfree(s->c128[i]); dfree(s->c64[i]); }
     for (auto &e : s->ev) if (e) cudaEventDestroy(e);
     for (auto &e : s->sw_ev) if (e) cudaEventDestroy(e);
@@ -1017,19 +1017,23 @@ int wust_solver_gauss_newton_product(wust_solver *s, const double *direction, do
 // ---------------------------------------------------------------------------
 // NCG update on the device (wust_reconstruct.m:24-57)
 // ---------------------------------------------------------------------------
-static double *ncg_partials(wust_solver *s) {
-    if (!s->ncg_part) s->ncg_part = dalloc<double>(3 * (size_t)kNcgMaxBlocks);
-    return s->ncg_part;
+static const NcgReduce &ncg_reduce(wust_solver *s) {
+    if (!s->ncg.part) {
+        s->ncg.part = dalloc<double>(3 * (size_t)kNcgMaxBlocks + 5);
+        s->ncg.result = s->ncg.part + 3 * (size_t)kNcgMaxBlocks;
+        s->ncg.ticket = reinterpret_cast<unsigned *>(s->ncg.result + 4);
+        WUST_CUDA(cudaMemsetAsync(s->ncg.ticket, 0, sizeof(double), s->st));
+    }
+    return s->ncg;
 }
-// Sum `per` values over nb block partials, in block order.
-static std::vector<double> ncg_sum(wust_solver *s, int nb, int per) {
-    std::vector<double> h((size_t)nb * per), out(per, 0.0);
-    WUST_CUDA(cudaMemcpyAsync(h.data(), s->ncg_part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, s->st));
-    WUST_CUDA(cudaStreamSynchronize(s->st));
-    for (int b = 0; b < nb; ++b)
-        for (int k = 0; k < per; ++k) out[k] += h[(size_t)b * per + k];
-    return out;
-}
+// The results of the launches before, once the stream has run them.
+struct NcgResult {
+    double v[4];
+    explicit NcgResult(wust_solver *s) {
+        WUST_CUDA(cudaMemcpyAsync(v, s->ncg.result, sizeof(v), cudaMemcpyDeviceToHost, s->st));
+        WUST_CUDA(cudaStreamSynchronize(s->st));
+    }
+};
 static double mean_step(const std::vector<double> &v) {
     double t = 0;
     for (size_t i = 1; i < v.size(); ++i) t += v[i] - v[i - 1];
@@ -1078,20 +1082,18 @@ int wust_ncg_direction(wust_solver *s, const double *roi, const double *z, const
         if (!s || !roi || !z || !prev_z || !direction || !beta_out || !gz_out)
             fail(WUST_ERR_INVALID_INPUT, "ncg_direction arguments missing");
         const size_t N = s->plane();
-        double *part = ncg_partials(s);
-        const std::vector<double> d2 = ncg_sum(s, ncg_dot2_launch(roi, z, prev_z, N, part, s->st), 2);
-        const double gz = d2[0];
-        double beta = 0.0;
-        if (same_frequency && prev_gz > 0) {
-            const double beta_fr = gz / prev_gz, beta_pr = d2[1] / prev_gz;
-            beta = std::min(std::max(beta_pr, 0.0), beta_fr);
-        }
-        std::vector<double> dd = ncg_sum(s, ncg_direction_launch(z, roi, beta, direction, N, part, s->st), 2);
-        if (dd[0] >= 0) {                         // not a descent direction: restart with -z
+        const NcgReduce &r = ncg_reduce(s);
+        ncg_dot2_launch(roi, z, prev_z, N, prev_gz, same_frequency != 0, r, s->st);
+        ncg_direction_launch(z, roi, false, direction, N, r, s->st);
+        NcgResult res(s);                         // gz, beta, g d, nonfinite entries
+        const double gz = res.v[0];
+        double beta = res.v[1];
+        if (res.v[2] >= 0) {                      // not a descent direction: restart with -z
             beta = 0.0;
-            dd = ncg_sum(s, ncg_direction_launch(z, roi, 0.0, direction, N, part, s->st), 2);
+            ncg_direction_launch(z, roi, true, direction, N, r, s->st);
+            res = NcgResult(s);
         }
-        if (dd[1] != 0 || !std::isfinite(gz) || gz < 0)
+        if (res.v[3] != 0 || !std::isfinite(gz) || gz < 0)
             fail(WUST_ERR_NUMERICAL_FAILURE, "Invalid preconditioned gradient");
         *beta_out = beta;
         *gz_out = gz;
@@ -1101,7 +1103,8 @@ int wust_ncg_direction(wust_solver *s, const double *roi, const double *z, const
 int wust_ncg_dot(wust_solver *s, const double *a, const double *b, double *out) {
     return guarded([&] {
         if (!s || !a || !b || !out) fail(WUST_ERR_INVALID_INPUT, "ncg_dot arguments missing");
-        *out = ncg_sum(s, ncg_dot_launch(a, b, s->plane(), ncg_partials(s), s->st), 1)[0];
+        ncg_dot_launch(a, b, s->plane(), ncg_reduce(s), s->st);
+        *out = NcgResult(s).v[0];
     });
 }
 
@@ -1112,12 +1115,12 @@ int wust_ncg_project(wust_solver *s, double *c, const double *direction, double 
         if (!s || !c || !direction || !update_mask) fail(WUST_ERR_INVALID_INPUT, "ncg_project arguments missing");
         if (!(c_min > 0 && c_max > c_min && max_update_mps > 0 && step_damping > 0 && std::isfinite(alpha)))
             fail(WUST_ERR_INVALID_INPUT, "Invalid speed bounds or step");
-        const std::vector<double> r = ncg_sum(
-            s, ncg_project_launch(c, direction, step_damping * alpha, max_update_mps, c_min, c_max, update_mask,
-                                  s->plane(), ncg_partials(s), s->st), 3);
-        if (r[0] != 0) fail(WUST_ERR_NUMERICAL_FAILURE, "Nonfinite slowness trial");
+        ncg_project_launch(c, direction, step_damping * alpha, max_update_mps, c_min, c_max, update_mask, s->plane(),
+                           ncg_reduce(s), s->st);
+        const NcgResult r(s);
+        if (r.v[0] != 0) fail(WUST_ERR_NUMERICAL_FAILURE, "Nonfinite slowness trial");
         if (relative_update)
-            *relative_update = std::sqrt(r[1]) / std::max(std::sqrt(r[2]), std::numeric_limits<double>::min());
+            *relative_update = std::sqrt(r.v[1]) / std::max(std::sqrt(r.v[2]), std::numeric_limits<double>::min());
     });
 }
 

@@ -112,13 +112,19 @@ void ncg_roi_launch(const double *g, const uint8_t *mask, double *roi, size_t n,
 void ncg_mask_scale_launch(double *z, const uint8_t *mask, double scale, size_t n, cudaStream_t st);
 void ncg_butterworth_launch(double2 *spec, int nx, int ny, double dx, double dy, double kc2, double order,
                             cudaStream_t st);
-// the launchers below return the number of block partials written
-int ncg_dot2_launch(const double *a, const double *b, const double *c, size_t n, double *part, cudaStream_t st);
-int ncg_dot_launch(const double *a, const double *b, size_t n, double *part, cudaStream_t st);
-int ncg_direction_launch(const double *z, const double *g, double beta, double *d, size_t n, double *part,
-                         cudaStream_t st);
-int ncg_project_launch(double *c, const double *d, double step, double max_update, double c_min, double c_max,
-                       const uint8_t *mask, size_t n, double *part, cudaStream_t st);
+// where the launchers below reduce to, one set per solver
+struct NcgReduce {
+    double *part;        // [3 kNcgMaxBlocks] block partials
+    unsigned *ticket;    // blocks that have arrived; zero between launches
+    double *result;      // [4]; [1] = beta, from dot2 to the direction
+};
+void ncg_dot2_launch(const double *a, const double *b, const double *c, size_t n, double prev_gz, bool conjugate,
+                     const NcgReduce &r, cudaStream_t st);
+void ncg_dot_launch(const double *a, const double *b, size_t n, const NcgReduce &r, cudaStream_t st);
+void ncg_direction_launch(const double *z, const double *g, bool restart, double *d, size_t n, const NcgReduce &r,
+                          cudaStream_t st);
+void ncg_project_launch(double *c, const double *d, double step, double max_update, double c_min, double c_max,
+                        const uint8_t *mask, size_t n, const NcgReduce &r, cudaStream_t st);
 
 // ---- prepare.cu (DTFT of the RF preparation) --------------------------------
 // time_s, freq: host; rf [nt, n_rx, n_tx] float or double, active [n_tx, n_rx]
