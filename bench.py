@@ -544,8 +544,7 @@ def run_simulate(args, torch):
     hpml = 20                                  # the Helmholtz grid's PML, cropped off
     c = p.c_true[hpml:-hpml, hpml:-hpml]
     x, y = p.x_m[hpml:-hpml], p.y_m[hpml:-hpml]
-    # the k-space PML outside the 512^2 model (552^2 with it; measured: a
-    # 32-cell PML, 576^2 = 2^6 3^2, ran 35 % slower through cuFFT)
+    # the k-space PML outside the 512^2 model (552^2 with it)
     pml = 20
     ny, nx = c.shape
     # the ring's grid points, moved into the cropped model grid
@@ -591,11 +590,11 @@ def run_simulate(args, torch):
     o.simulate(c, float(y[1] - y[0]), float(x[1] - x[0]), dt, src[:20], tx[:1], rx, pml, c_ref, 1000.0)
     cpu_s = time.perf_counter() - t0
     Ny, Nx = ny + 2 * pml, nx + 2 * pml
-    # per transmitter and time step: 7 FFT passes (R2C of p, C2R and R2C of
-    # the two velocities, C2R of the two divergences) read and write at
-    # least one real plane each, the three pointwise kernels 11 planes
+    # per transmitter and time step: the four kernels read and write the
+    # spectra of the pressure, the gradients, the velocities and the
+    # divergence, and the velocity and density fields
     plane = Ny * Nx * 4
-    alg_bytes = (7 * 2 + 11) * plane
+    alg_bytes = 22 * plane
     achieved = alg_bytes * units / (ms * 1e-3) / 1e9
     peaks = {}
     try:
@@ -613,7 +612,7 @@ def run_simulate(args, torch):
                     l2=f"fields {7 * tx.size * plane / 1e9:.1f} GB, larger than L2"),
         e2e=dict(value=units / e2e_s, unit="tx*steps/s", h2d_bytes_per_step=int(cm.nbytes + src.nbytes),
                  d2h_bytes_per_step=int(rec["pressure"].nbytes)),
-        roofline=dict(kernel="time step (cuFFT R2C/C2R + 3 fused pointwise kernels) over all transmitters", bound="hbm",
+        roofline=dict(kernel="time step (fused_x_kernel and fused_y_kernel, twice each) over all transmitters", bound="hbm",
                       achieved=achieved, peak=hbm, unit="GB/s", frac=achieved / hbm,
                       peak_source="MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6650 GB/s", traffic=None,
                       algorithmic_bytes_per_tx_step=alg_bytes),
@@ -687,7 +686,7 @@ def run_dtft(args, torch):
                     l2="RF 512 MB, larger than L2"),
         e2e=dict(value=1e3 / e2e_ms, unit="preparations/s", h2d_bytes_per_step=rf_bytes,
                  d2h_bytes_per_step=n_f * n_rx * n_tx * 8),
-        roofline=dict(kernel="dtft_kernel (FP64 CUDA-core GEMM, RF streamed once)", bound="hbm", achieved=achieved,
+        roofline=dict(kernel="dtft_fold_kernel (FP64 matrix instruction, RF streamed once)", bound="hbm", achieved=achieved,
                       peak=hbm, unit="GB/s", frac=achieved / hbm,
                       peak_source="MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6650 GB/s", traffic=None),
         cpu_baseline=dict(value=1.0 / cpu_s, unit="preparations/s", cores=1, kind="port",

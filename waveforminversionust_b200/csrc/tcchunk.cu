@@ -325,9 +325,9 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
         // a lane takes one 16-byte unit of one source, a warp 4 units of 8
         // sources, 512 bytes of a packed chunk in a row, straight from registers.
         // Loops stay rolled: a step runs all of its code once, and straight-line
-        // code for 8 sources was bound by instruction fetch (produce at 16
-        // sources 2.5 us, here 0.8; at 128 4.5 against 2.7 without fields).
-        // Per step of 256 sources 8.6 -> 9.0 us with fields, 192 without 5.2 -> 4.5.
+        // code for 8 sources was bound by instruction fetch.  Per step of 16
+        // sources 2.5 -> 0.8 us, of 64 (half of the steps with fields) 3.5 -> 2.8,
+        // of 192 without fields 5.2 -> 4.6; of 256 with fields 8.6 -> 9.0.
         constexpr int RPC = BF ? kCkRowsPerChunk16 : kCkRowsPerChunk;
         constexpr int RPU = RPC / 8, NI = 16 / RPU;                   // rows of a 16-byte unit; items of 8 sources
         if (fields) {
@@ -590,13 +590,13 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
     // so none waits on another's latency.  Chunk ci's stage is slot ci %
     // stages, used for the (ci / stages)-th time; each thread counts its slots
     // and phases along.  Up to N = 128 the ring is bound by what these threads
-    // do per stage rather than by bytes or products: with divisions by kc and
+    // do per stage rather than by bytes or products.  With divisions by kc and
     // the ring's length per chunk, and the timer read in each wait, a step's
-    // ring took 13.3 us at 552^2 (TF32 and BF16 steps of 256 sources averaged),
-    // 9.9 at 437 x 401 and 6.6 at 288^2 (128 sources), 12.0, 9.1 and 6.0 in the
-    // boundary chain; now 9.7, 5.9, 3.9 and 7.5, 5.3, 3.6.  An L2 prefetch of the
-    // next step's pages while the MMAs' results are finished: TF32 steps 4 %
-    // slower.
+    // ring took 13.3 us at 552^2 (256 sources, TF32 and BF16 steps averaged),
+    // 9.9 at 437 x 401 (97) and 6.6 at 288^2 (64), and 12.0, 9.1 and 6.0 in the
+    // boundary chain (16); now 11.0, 6.3 and 3.7, and 5.8, 4.6 and 3.4.  An L2
+    // prefetch of the next step's pages while this one's results are finished:
+    // TF32 steps 4 % slower.
     int c_slot = 0, c_q = 0, a_k = 0;                            // a copy thread's next chunk; thread 0: the next MMAs
     uint32_t c_next = 0, c_phase = 0;
     const uint8_t *a_src = nullptr;
