@@ -51,3 +51,39 @@ def test_simulation_matches_the_oracle(tmp_path, ny, nx, pml, n_tx, tx_batch, q,
     want = np.transpose(ref, (2, 0, 1))
     assert got.shape == want.shape
     assert np.linalg.norm(got - want) < 1.2e-4 * np.linalg.norm(want)
+
+
+def test_threads_with_grids_of_different_sizes(tmp_path):
+    """Calls from several threads, each with a grid of its own, give what they
+    give one after another."""
+    import threading
+    import torch
+    from waveforminversionust_b200.simulate import wust_simulate
+    t = np.arange(12) * 60e-9
+    src = np.sin(2 * np.pi * .8e6 * t)
+
+    def call(ny, nx, stream):
+        model = dict(c_mps=np.full((ny, nx), 1500.0), x_m=np.arange(nx) * .5e-3, y_m=np.arange(ny) * .5e-3,
+                     tx_index=np.array([5, 9]), rx_index=np.array([ny * nx - 3]), dt_s=60e-9, source_pressure=src)
+        cfg = dict(backend="native-batch", pml_size=6, density_kg_m3=1000, sound_speed_ref_mps=1550, downsample_factor=1,
+                   time_offset_s=0, work_dir=str(tmp_path))
+        return wust_simulate(model, cfg, stream=stream)["pressure"]
+
+    sizes = [(12, 14), (100, 116), (228, 244), (52, 54), (180, 276)]
+    want = [call(*s, None) for s in sizes]
+    wrong = []
+
+    def run(k):
+        stream = torch.cuda.Stream()
+        for _ in range(6):
+            try:
+                if not np.array_equal(call(*sizes[k], stream), want[k]):
+                    wrong.append((sizes[k], "differs"))
+            except Exception as e:                                        # noqa: BLE001
+                wrong.append((sizes[k], e))
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(len(sizes))]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not wrong

@@ -626,6 +626,7 @@ static std::vector<float> decimation_taps(int q, int half_length, double beta) {
 }
 
 // ---- the fused steps: workspace layout and host side ---------------------------
+constexpr size_t kFusedSmem = 226 * 1024;        // dynamic; the plans take another 0.7 KB
 struct FusedLayout {
     FusedGeom g;
     int KT;                        // ky columns per x tile
@@ -649,7 +650,7 @@ static FusedLayout fused_layout(int ny, int nx, int pml, int ntx, int nrx, int n
     if ((long long)g.Nx * g.Ny <= 1 << 17)
         for (int C = 8; C >= 1; C /= 2) {
             const ResidentShape m = resident_shape(g.Ny, g.Nx, C);
-            if (m.bytes > 225 * 1024) break;
+            if (m.bytes > kFusedSmem) break;
             L.resident = true;
             L.shape = m;
             if (C * g.S <= 120) break;
@@ -704,7 +705,7 @@ static bool fused_fits(const FusedLayout &L) {
             }
         return std::max(p, n);
     };
-    return L.smem_x <= 226 * 1024 && L.smem_p <= 226 * 1024 && std::max(L.g.Nx, L.g.Ny) <= 32767 &&
+    return L.smem_x <= kFusedSmem && L.smem_p <= kFusedSmem && std::max(L.g.Nx, L.g.Ny) <= 32767 &&
            L.g.cells <= 2147483647ULL && L.g.S <= 65535 &&
            std::max(largest_prime(L.g.Nx), largest_prime(L.g.Ny)) <= (L.resident ? 113 : 37);
 }
@@ -791,18 +792,20 @@ static void simulate_fused(const SimulateArgs &a, const FusedLayout &L, uint8_t 
         (float2 *)(ws + L.twy));
     ++g_kernel_launches;
     WUST_LAUNCH_CHECK();
-    auto grow = [](const void *kernel, size_t bytes) {
-        WUST_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    // to the limit, not to this grid's need: the attribute belongs to the
+    // function, and another thread may be launching it at another size
+    auto grow = [](const void *kernel) {
+        WUST_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFusedSmem));
     };
     auto x_first = L.KT == 8 ? fused_x_kernel<true, 3> : fused_x_kernel<true, 2>;
     auto x_second = L.KT == 8 ? fused_x_kernel<false, 3> : fused_x_kernel<false, 2>;
     if (L.resident) {
-        grow((const void *)fused_resident_kernel, L.shape.bytes);
+        grow((const void *)fused_resident_kernel);
     } else {
-        grow((const void *)x_first, L.smem_x);
-        grow((const void *)x_second, L.smem_x);
-        grow((const void *)fused_y_kernel<true>, L.smem_v);
-        grow((const void *)fused_y_kernel<false>, L.smem_p);
+        grow((const void *)x_first);
+        grow((const void *)x_second);
+        grow((const void *)fused_y_kernel<true>);
+        grow((const void *)fused_y_kernel<false>);
     }
     float *record = (float *)(ws + L.record);
     float2 *u = (float2 *)(ws + L.fields), *r = u + (size_t)S * g.cells;

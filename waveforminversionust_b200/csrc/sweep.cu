@@ -644,6 +644,11 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
     }
 }
 
+// Dynamic shared memory of any plan at most.  The kernels' attribute is set to
+// this, not to the plan's: it belongs to the function, and another thread may
+// be launching the same shape at another size.
+constexpr size_t kSweepClusterSmem = 232448 - 1024;
+
 // How a solve is split: cl CTAs per cluster, shape index; cl == 0: none fits.
 struct SweepPlan {
     int cl, shape, RB, clusters, stages;
@@ -695,8 +700,8 @@ static SweepPlan sweep_plan(int ny, int S, int max_ctas) {
             if (RB > TR || RB * (z.cl - 1) >= n || 2 * n > (s == 0 ? 5 : 6) * CT) continue;
             int stages = 4;
             size_t smem = sweep_shape_bytes<ADJ>(s, ny, stages);
-            while (smem > 232448 - 1024 && stages > 2) smem = sweep_shape_bytes<ADJ>(s, ny, --stages);
-            if (smem > 232448 - 1024) continue;
+            while (smem > kSweepClusterSmem && stages > 2) smem = sweep_shape_bytes<ADJ>(s, ny, --stages);
+            if (smem > kSweepClusterSmem) continue;
             const int clusters = ceil_div(S, NS);
             const double fma = 1.3 * 4.0 * TR * NS * n / 128.0, rows = 8.0 * RB * n / 45.0;
             const double t = (double)ceil_div(clusters, at_once) * (std::max(fma, rows) + 25.0 * n * NS / CT + 3000.0);
@@ -760,7 +765,7 @@ static bool sweep_cluster_solve(const Coefs<float2> &co, const float2 *invT, con
     p.RB = g.RB;
     p.stages = g.stages;
     const void *kernel = sweep_shape_kernel<ADJ>(g.shape);
-    WUST_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+    WUST_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepClusterSmem));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(g.clusters * g.cl);
     cfg.blockDim = dim3(CT);
