@@ -186,11 +186,12 @@ struct NsParams {
     unsigned long long timeout_ns;
 };
 
+// Grid barrier; the release is cumulative over the CTA's writes (552^2: 22.06 ms
+// with a gpu-scope fence before it, 21.72 without).
 __device__ __forceinline__ bool ns_sync(unsigned *ctr, unsigned target, int *err, int *s_ok,
                                         unsigned long long timeout_ns) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        asm volatile("fence.acq_rel.gpu;" ::: "memory");
         asm volatile("fence.proxy.async.global;" ::: "memory");
         asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(ctr), "r"(1u) : "memory");
         int ok = 1;
