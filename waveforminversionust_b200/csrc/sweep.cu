@@ -251,13 +251,12 @@ struct SweepShape {
     static constexpr int ITEMS = RW * NSW > 16 ? 5 : 6;      // stencil items per thread: 2 n <= ITEMS * CT
     static constexpr int NSP = NS > 2 ? NS + 2 : NS;         // entries per row of B: rows of a quarter-warp in distinct banks
     static constexpr int PS = NS * TR + 2;                   // entries per partial tile, likewise
-    // K of a warp (H: an eighth) in whole stages; the rows of B beyond n are zero
+    // K of a warp (H: an eighth) in whole stages
     __host__ __device__ static int kper(int n) { return ADJ ? (n + SK - 1) / SK * SK : ((n + CW - 1) / CW + SK - 1) / SK * SK; }
-    __host__ __device__ static int kpad(int n) { return ADJ ? kper(n) : CW * kper(n); }
     __host__ __device__ static int ldc(int ny) { return (ny + 3) / 2 * 2; }
     __host__ __device__ static size_t col(int ny) { return sizeof(float2) * (size_t)NS * ldc(ny); }
     __host__ __device__ static size_t work(int n) {          // B, or the partial tiles
-        const size_t b = sizeof(float2) * (size_t)kpad(n) * NSP, q = sizeof(float2) * (size_t)CW * PS;
+        const size_t b = sizeof(float2) * (size_t)n * NSP, q = sizeof(float2) * (size_t)CW * PS;
         return b > q ? b : q;
     }
     __host__ __device__ static size_t ring(int ny) { return (col(ny) + work(ny - 2) + 127) / 128 * 128; }
@@ -444,7 +443,6 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
                     if (h * HS + q < ns) uo[plane * q] = b[q];
             }
         }
-        for (int e = tid; e < (Sh::kpad(n) - n) * NSP; e += CT) X[(size_t)n * NSP + e] = f2(0.f, 0.f);
         if (wu && j >= 2) {
             // rows 0 and ny - 1 of u(:, j - 1), which no page reads
             for (int e = tid; e < 2 * ns; e += CT) {
@@ -543,6 +541,9 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
                 slot = 0;
                 phase ^= 1u;
             }
+            // K of this stage: a box also holds the page's border and entries of its neighbours beyond n, which nobody
+            // has said are finite
+            const int left = n - (ADJ ? 0 : k_own) - g * SK;
             // column q of the stage: its box, its row, and the entry that the copy put in front of it or not
             auto column = [&](int q, int off) -> const float2 * {
                 return reinterpret_cast<const float2 *>(stage + (q & 1) * Sh::box_at) + (q >> 1) * INN +
@@ -553,8 +554,7 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
                 const float2 *Ar[RW];
 #pragma unroll
                 for (int x = 0; x < RW; ++x) Ar[x] = column(trow(x) - Sh::WR * warp, g * SK + 1) + part;
-#pragma unroll
-                for (int kk = 0; kk < SK; kk += 8) {
+                auto product = [&](int kk) {
                     float2 b[NSW];
                     load_pairs(b, Bs + kk * NSP);
 #pragma unroll
@@ -563,12 +563,18 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
 #pragma unroll
                         for (int y = 0; y < NSW; ++y) cfma_conj(acc[x][y], a, b[y]);
                     }
+                };
+                if (left >= SK) {
+#pragma unroll
+                    for (int kk = 0; kk < SK; kk += 8) product(kk);
+                } else {
+#pragma unroll 1
+                    for (int kk = 0; kk < left - part; kk += 8) product(kk);
                 }
             } else {
                 const float2 *Bs = X + (size_t)(k_own + g * SK) * NSP + tsrc;
                 const float2 *A0 = column(0, r0 + 1) + trow(0), *A1 = column(1, r0 + 1) + trow(0);   // SK is even
-#pragma unroll
-                for (int kk = 0; kk < SK; ++kk) {
+                auto product = [&](int kk) {
                     const float2 *Ak = (kk & 1 ? A1 : A0) + (kk >> 1) * INN;
                     float2 b[NSW];
                     load_pairs(b, Bs + kk * NSP);
@@ -578,6 +584,13 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
 #pragma unroll
                         for (int y = 0; y < NSW; ++y) cfma(acc[x][y], a, b[y]);
                     }
+                };
+                if (left >= SK) {
+#pragma unroll
+                    for (int kk = 0; kk < SK; ++kk) product(kk);
+                } else {
+#pragma unroll 1
+                    for (int kk = 0; kk < left; ++kk) product(kk);
                 }
             }
         }
