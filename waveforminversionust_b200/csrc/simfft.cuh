@@ -400,7 +400,7 @@ __device__ __forceinline__ void stage_prime(int z, const Lines &lines, const Fft
         float2 a[KT][CT], s[KT][CT], sum[CT];
         int idx[KT];
 #pragma unroll
-        for (int c = 0; c < CT; ++c) sum[c] = base[c * next];
+        for (int c = 0; c < CT; ++c) sum[c] = on ? base[c * next] : make_float2(0.f, 0.f);   // others are writing elsewhere
 #pragma unroll
         for (int t = 0; t < KT; ++t) {
             idx[t] = 0;
