@@ -1148,21 +1148,14 @@ int wust_dtft_ws(const double *time_s, int n_time, const double *frequencies_hz,
         if (workspace && (workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255) != 0))
             fail(WUST_ERR_INVALID_INPUT, "dtft workspace of %zu bytes on 256 required", need);
         cudaStream_t st = static_cast<cudaStream_t>(stream);
-        // freed on every way out
-        struct Own {
-            void *p = nullptr;
-            cudaStream_t st;
-            ~Own() { if (p) cudaFreeAsync(p, st); }
-        } own{nullptr, st};
-        if (!workspace) {
-            WUST_CUDA(cudaMallocAsync(&own.p, need, st));
-            workspace = own.p;
-        }
+        CallMemory mem(st);
+        workspace = mem.take(workspace, need);
         int *bad = nullptr, h_bad = 0;
         dtft_launch(time_s, frequencies_hz, n_time, n_f, dt, rf, rf_is_double != 0, n_rx, n_tx, active, workspace,
                     reinterpret_cast<float2 *>(Y), &bad, st);
         WUST_CUDA(cudaMemcpyAsync(&h_bad, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
         WUST_CUDA(cudaStreamSynchronize(st));
+        mem.done = true;
         if (h_bad) fail(WUST_ERR_INVALID_INPUT, "Nonfinite RF on an active channel");
     });
 }

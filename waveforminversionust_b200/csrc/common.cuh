@@ -31,6 +31,29 @@ void set_last_error(const std::string &msg);
 
 #define WUST_LAUNCH_CHECK() WUST_CUDA(cudaPeekAtLastError())
 
+// Device memory of one call on a stream: the caller's, or a block of the
+// call's own.  A call that ends in an error may have queued work that still
+// uses it: the stream is waited for on that way out too, before anybody takes
+// the memory (or the outputs) for free.
+struct CallMemory {
+    cudaStream_t st;
+    void *own = nullptr;
+    bool done = false;       // the call has waited for its work
+    explicit CallMemory(cudaStream_t stream) : st(stream) {}
+    CallMemory(const CallMemory &) = delete;
+    ~CallMemory() {
+        if (!done) cudaStreamSynchronize(st);
+        if (own) cudaFreeAsync(own, st);
+    }
+    // the caller's block, or `bytes` of its own
+    void *take(void *given, size_t bytes) {
+        if (given) return given;
+        void *block = nullptr;
+        WUST_CUDA(cudaMallocAsync(&block, bytes, st));
+        return own = block;
+    }
+};
+
 // ---------------------------------------------------------------------------
 // Complex arithmetic (interleaved float2 / double2).
 // ---------------------------------------------------------------------------

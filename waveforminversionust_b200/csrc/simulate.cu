@@ -869,17 +869,9 @@ void simulate_rf(const SimulateArgs &a, void *workspace, float *rf, cudaStream_t
         simulate_library(a, rf, st);
         return;
     }
-    // freed on every way out
-    struct Own {
-        void *p = nullptr;
-        cudaStream_t st;
-        ~Own() { if (p) cudaFreeAsync(p, st); }
-    } own{nullptr, st};
-    if (!workspace) {
-        WUST_CUDA(cudaMallocAsync(&own.p, L.total, st));
-        workspace = own.p;
-    }
-    simulate_fused(a, L, static_cast<uint8_t *>(workspace), rf, st);
+    CallMemory mem(st);
+    simulate_fused(a, L, static_cast<uint8_t *>(mem.take(workspace, L.total)), rf, st);
+    mem.done = true;
 }
 
 // Grids beyond the fused kernels (fused_fits): library transforms.
