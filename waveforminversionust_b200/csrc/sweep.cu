@@ -232,6 +232,7 @@ struct __align__(64) SweepClusterParams {
     SrcView src;
     int *err;
     int ny, nx, S, n, RB, stages;
+    int s0;             // first source of the launch
     unsigned long long timeout_ns;
     CUtensorMap pages;  // invT as rows of two page columns, a box of one parity of a stage's columns
 };
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
     unsigned rank, ncta;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ncta));
-    const int s_first = (int)(blockIdx.x / ncta) * NS, ns = min(NS, p.S - s_first);
+    const int s_first = p.s0 + (int)(blockIdx.x / ncta) * NS, ns = min(NS, p.S - s_first);
     const int r0 = (int)rank * p.RB, rows = min(p.RB, n - r0);             // interior rows r0 .. r0 + rows - 1
     const size_t page_sz = (size_t)ny * ny, plane = (size_t)ny * nx;
     const int steps = 2 * (nx - 1);
@@ -662,9 +663,10 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
 // be launching the same shape at another size.
 constexpr size_t kSweepClusterSmem = 232448 - 1024;
 
-// How a solve is split: cl CTAs per cluster, shape index; cl == 0: none fits.
+// How a solve is split: cl CTAs per cluster, shape index, clusters in all and
+// in one launch; cl == 0: none fits.
 struct SweepPlan {
-    int cl, shape, RB, clusters, stages;
+    int cl, shape, RB, clusters, per_launch, stages;
     size_t smem;
 };
 constexpr int kSweepShapes[][2] = {{6, 6}, {4, 4}, {3, 4}, {2, 2}, {1, 1}};    // RW, NSW
@@ -694,9 +696,11 @@ static const void *sweep_shape_kernel(int shape) {
 // The shape with the least estimated time per step.  How many clusters of a
 // size run at once is the B200's (148 SMs, clusters inside a GPC, one CTA per
 // SM); a wrong count costs time, not correctness: the clusters do not wait on
-// each other.  Clocks per step: the multiply-adds at 128 per clock (1.3 of
-// that as measured) or the page rows at 45 bytes per clock, the stencil of
-// all rows, and 3000 for the sums, the exchange and the barriers.
+// each other.  A cap of max_ctas CTAs is kept by launches of as many clusters
+// as it holds, one after another on the stream.  Clocks per step: the
+// multiply-adds at 128 per clock (1.3 of that as measured) or the page rows at
+// 45 bytes per clock, the stencil of all rows, and 3000 for the sums, the
+// exchange and the barriers.
 template <bool ADJ>
 static SweepPlan sweep_plan(int ny, int S, int max_ctas) {
     struct { int cl, at_once; } const sizes[] = {{1, 148}, {2, 70}, {4, 33}, {6, 22}, {8, 15}};
@@ -719,7 +723,7 @@ static SweepPlan sweep_plan(int ny, int S, int max_ctas) {
             const double fma = 1.3 * 4.0 * TR * NS * n / 128.0, rows = 8.0 * RB * n / 45.0;
             const double t = (double)ceil_div(clusters, at_once) * (std::max(fma, rows) + 25.0 * n * NS / CT + 3000.0);
             if (best.cl == 0 || t < best_t) {
-                best = SweepPlan{z.cl, s, RB, clusters, stages, smem};
+                best = SweepPlan{z.cl, s, RB, clusters, max_ctas > 0 ? std::min(clusters, at_once) : clusters, stages, smem};
                 best_t = t;
             }
         }
@@ -780,7 +784,6 @@ static bool sweep_cluster_solve(const Coefs<float2> &co, const float2 *invT, con
     const void *kernel = sweep_shape_kernel<ADJ>(g.shape);
     WUST_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepClusterSmem));
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(g.clusters * g.cl);
     cfg.blockDim = dim3(CT);
     cfg.dynamicSmemBytes = g.smem;
     cfg.stream = st;
@@ -792,8 +795,12 @@ static bool sweep_cluster_solve(const Coefs<float2> &co, const float2 *invT, con
     cfg.attrs = at;
     cfg.numAttrs = 1;
     void *args[] = {&p};
-    WUST_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
-    ++g_kernel_launches;
+    for (int c = 0; c < g.clusters; c += g.per_launch) {
+        cfg.gridDim = dim3(std::min(g.per_launch, g.clusters - c) * g.cl);
+        p.s0 = c * 2 * kSweepShapes[g.shape][1];
+        WUST_CUDA(cudaLaunchKernelExC(&cfg, kernel, args));
+        ++g_kernel_launches;
+    }
     WUST_LAUNCH_CHECK();
     return true;
 }
