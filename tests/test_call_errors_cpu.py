@@ -74,6 +74,17 @@ cudaError_t cudaFreeAsync(void *p, cudaStream_t) {
     ++freed;
     return cudaSuccess;
 }
+cudaError_t cudaMalloc(void **p, size_t) {
+    *p = (void *)0x600000;
+    if (++calls == fail_at) return last = cudaErrorMemoryAllocation;
+    ++taken;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void *p) {
+    if (p != (void *)0x600000 || pending) wrong("freed what is not its own, or in use");
+    ++freed;
+    return cudaSuccess;
+}
 cudaError_t cudaPeekAtLastError() { return last; }
 cudaError_t cudaGetLastError() { const cudaError_t e = last; last = cudaSuccess; return e; }
 const char *cudaGetErrorString(cudaError_t) { return "made up"; }
@@ -81,10 +92,10 @@ const char *cudaGetErrorString(cudaError_t) { return "made up"; }
 
 static std::vector<double> c, source, t, f;
 static std::vector<int> tx, rx;
-static int ny, nx, nt = 6, q;
+static int ny, nx, nt = 6, q, batch;
 static int simulate(void *ws, size_t bytes) {
     return wust_simulate_ws(c.data(), ny, nx, 1e-3, 1e-3, 1e-7, nt, source.data(), tx.data(), (int)tx.size(), rx.data(),
-                            (int)rx.size(), 4, 1600, 1000, q, 1, (float *)0x300000, ws, bytes, kStream);
+                            (int)rx.size(), 4, 1600, 1000, q, batch, (float *)0x300000, ws, bytes, kStream);
 }
 static int dtft(void *ws, size_t bytes) {
     return wust_dtft_ws(t.data(), (int)t.size(), f.data(), (int)f.size(), (void *)0x300000, 0, 3, 5, (uint8_t *)0x400000,
@@ -109,16 +120,19 @@ static void every_failure(const char *name, int (*call)(void *, size_t), size_t 
     }
 }
 int main() {
-    const int grids[][3] = {{11, 13, 1}, {240, 232, 1}, {240, 232, 3}};
+    // a cluster's grid, tiles, their records decimated, and fields that a pool does not hold
+    const int grids[][4] = {{11, 13, 1, 1}, {240, 232, 1, 1}, {240, 232, 3, 1}, {512, 504, 1, 0}};
     for (const auto &g : grids) {
         ny = g[0];
         nx = g[1];
         q = g[2];
+        batch = g[3];
         c.assign((size_t)ny * nx, 1500.0);
         source.assign(nt, 1.0);
         tx = {3, 8};
+        for (int i = 0; !batch && i < 10; ++i) tx.push_back(20 + i);
         rx = {5, 9, 70};
-        const size_t bytes = wust_simulate_workspace_bytes(ny, nx, 4, (int)tx.size(), (int)rx.size(), nt, q, 1);
+        const size_t bytes = wust_simulate_workspace_bytes(ny, nx, 4, (int)tx.size(), (int)rx.size(), nt, q, batch);
         if (!bytes) wrong("not the path meant");
         every_failure("simulate", simulate, bytes);
     }

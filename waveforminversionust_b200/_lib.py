@@ -119,3 +119,27 @@ def check(status: int) -> None:
     if status != WUST_OK:
         msg = load().wust_last_error().decode(errors="replace")
         raise WustError(status, msg)
+
+
+# Largest block that a call borrows from torch's allocator, which keeps what it gets back.
+WORKSPACE_LIMIT = 64 << 20
+
+
+def workspace(need: int, stream):
+    """Device memory of one call on ``stream``: a block of torch's allocator and its first 256-byte boundary.
+
+    The library's own allocation maps and unmaps memory on every call (0.4 to 0.8 ms, more than the DTFT of a full
+    array's records takes), but gives it back when the call is over; torch keeps it, out of reach of a solver that the
+    library allocates later.  So only blocks of up to WORKSPACE_LIMIT come from torch; larger ones belong to calls of
+    tens of milliseconds.  (None, None) for those, for streams that torch does not know and where torch has no memory:
+    the library allocates, or says that it cannot.
+    """
+    import torch
+    if not 0 < need <= WORKSPACE_LIMIT or not isinstance(stream, torch.cuda.Stream):
+        return None, None
+    try:
+        with torch.cuda.stream(stream):
+            block = torch.empty(need + 256, dtype=torch.uint8, device="cuda")
+    except torch.OutOfMemoryError:
+        return None, None
+    return block, C.c_void_p(-(-block.data_ptr() // 256) * 256)

@@ -34,22 +34,28 @@ void set_last_error(const std::string &msg);
 // Device memory of one call on a stream: the caller's, or a block of the
 // call's own.  A call that ends in an error may have queued work that still
 // uses it: the stream is waited for on that way out too, before anybody takes
-// the memory (or the outputs) for free.
+// the memory (or the outputs) for free.  A block of its own goes back when the
+// call is over: to the stream's pool, or, above kPoolBytes, straight to the
+// device (the pool maps a block piece by piece, 13 us per MB; cudaMalloc and
+// cudaFree take 0.7 ms together up to 64 MB and 1.4 for 550).
 struct CallMemory {
+    static constexpr size_t kPoolBytes = 64 << 20;
     cudaStream_t st;
     void *own = nullptr;
+    bool pooled = false;
     bool done = false;       // the call has waited for its work
     explicit CallMemory(cudaStream_t stream) : st(stream) {}
     CallMemory(const CallMemory &) = delete;
     ~CallMemory() {
         if (!done) cudaStreamSynchronize(st);
-        if (own) cudaFreeAsync(own, st);
+        if (own) pooled ? cudaFreeAsync(own, st) : cudaFree(own);
     }
     // the caller's block, or `bytes` of its own
     void *take(void *given, size_t bytes) {
         if (given) return given;
         void *block = nullptr;
-        WUST_CUDA(cudaMallocAsync(&block, bytes, st));
+        pooled = bytes <= kPoolBytes;
+        WUST_CUDA(pooled ? cudaMallocAsync(&block, bytes, st) : cudaMalloc(&block, bytes));
         return own = block;
     }
 };

@@ -93,15 +93,11 @@ def dtft_device(time_s, frequencies_hz, pressure, active, stream=None):
     Y = torch.empty((f.size, n_rx, n_tx), dtype=torch.complex64, device=dev)
     st = stream if stream is not None else torch.cuda.current_stream()
     lib = _lib.load()
-    # the tables' room from torch's allocator: the library's own allocation maps and unmaps memory on every call.
-    # The call has synchronized the stream when it returns, so the block may go back at once.
     need = lib.wust_dtft_workspace_bytes(t.size, f.size)
-    with torch.cuda.stream(st):
-        ws = torch.empty(need + 256, dtype=torch.uint8, device=dev)
-    at = -(-ws.data_ptr() // 256) * 256
+    ws, at = _lib.workspace(need, st)                # the call synchronizes the stream: the block may go back after it
     check(lib.wust_dtft_ws(t.ctypes.data_as(C.c_void_p), t.size, f.ctypes.data_as(C.c_void_p), f.size,
                            C.c_void_p(p.data_ptr()), int(is_double), n_rx, n_tx, C.c_void_p(act.data_ptr()),
-                           C.c_void_p(Y.data_ptr()), C.c_void_p(at), need, C.c_void_p(st.cuda_stream)))
+                           C.c_void_p(Y.data_ptr()), at, need, C.c_void_p(st.cuda_stream)))
     return Y.permute(2, 1, 0)
 
 

@@ -101,17 +101,8 @@ def wust_simulate(model: dict, cfg: dict, stream=None) -> dict:
     batch = 0 if cfg["backend"] == "native-batch" else 1
     if "tx_batch" in cfg:
         batch = int(cfg["tx_batch"])
-    # the fields' room from torch's allocator: the library's own allocation maps and unmaps memory on every call.
-    # The call has synchronized the stream when it returns, so the block may go back at once.
     need = lib.wust_simulate_workspace_bytes(ny, nx, pml, n_tx, n_rx, n_time, q, batch)
-    ws = None
-    if need:
-        with torch.cuda.stream(st):
-            try:
-                ws = torch.empty(need + 256, dtype=torch.uint8, device="cuda")
-            except torch.OutOfMemoryError:            # the library reports what it cannot allocate
-                pass
-    at = C.c_void_p(-(-ws.data_ptr() // 256) * 256) if ws is not None else None
+    ws, at = _lib.workspace(need, st)                 # the call synchronizes the stream: the block may go back after it
     t0 = time.perf_counter()
     check(lib.wust_simulate_ws(cm.ctypes.data_as(C.c_void_p), ny, nx, dy, dx, dt, n_time, src.ctypes.data_as(C.c_void_p),
                                ti.ctypes.data_as(C.c_void_p), n_tx, ri.ctypes.data_as(C.c_void_p), n_rx, pml, c_ref,
