@@ -747,7 +747,10 @@ __global__ void __launch_bounds__(FT, 1) factor_flow_kernel(FlowParams p) {
                         });
                 }
             }
-            if (__syncthreads_or(!ok)) return;
+            if (__syncthreads_or(!ok)) {
+                asm volatile("cp.async.wait_all;" ::: "memory");           // the next page's coefficients
+                return;
+            }
             // row panel slice R[u][cl] = (P A[K, .])_{u, c0+cl}; R = P on the columns of K.  8 x 24 threads, 2 x 2
             // entries each: shared memory delivers 128 bytes per clock to the registers, broadcast or not, which
             // bounds narrower splits; fewer threads with more entries are bound by the issue of their few warps
@@ -848,7 +851,10 @@ __global__ void __launch_bounds__(FT, 1) factor_flow_kernel(FlowParams p) {
                     if (r < n && c < n) p.invT[(size_t)j * page_sz + (size_t)(r + 1) + (size_t)ny * (c + 1)] = a[i][jj];
                 }
         }
-        if (!grid_barrier(p.counter, p.err, gridDim.x, epoch, p.timeout_ns, 5004)) return;
+        if (!grid_barrier(p.counter, p.err, gridDim.x, epoch, p.timeout_ns, 5004)) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            return;
+        }
     }
 }
 

@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
     // stages per step: H skips what lies beyond n
     const int k_own = warp * kper, per = ADJ ? kper / SK : max(0, min(kper, n - k_own) + SK - 1) / SK;
     int f_step = per ? 0 : steps, f_g = 0, f_slot = 0;
-    bool alive = true;
+    int lost = 0;                                                          // stages from an expired wait to the end
     auto page_at = [&](int i) {                                            // first column of the page, of all pages
         bool fwd;
         const int j = step_col(i, nx, fwd);
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
     };
     auto fetch = [&]() {
         if (f_step >= steps) return;
-        if (lane == 0 && alive) {
+        if (lane == 0 && !lost) {
             const int first = page_at(f_step) + 1 + (ADJ ? r0 + Sh::WR * warp : k_own + f_g * SK);
             const int off = ADJ ? f_g * SK + 1 : r0 + 1;
             tc::mbar_expect_tx(full + f_slot, 2 * Sh::box);
@@ -531,8 +531,8 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
         const int col0 = page_at(i) + 1 + (ADJ ? r0 + Sh::WR * warp : k_own);  // of this warp's columns
 #pragma unroll 1
         for (int g = 0; g < per; ++g) {
-            if (alive && !tc::mbar_wait(full + slot, phase, p.timeout_ns)) {
-                alive = false;
+            if (!lost && !tc::mbar_wait(full + slot, phase, p.timeout_ns)) {
+                lost = (steps - i) * per - g;
                 atomicCAS(p.err, 0, SITE_COPY);
             }
             __syncwarp();                                  // this stage has landed, the one before it is consumed
@@ -655,6 +655,12 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
         }
         __syncthreads();
         asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
+    // after an expired wait: the copies issued ahead of it land (bounded) before the block ends
+    if (lane == 0 && lost) {
+        const int first = steps * per - lost;
+        for (int c = first; c < first + min(p.stages - 1, lost); ++c)
+            tc::mbar_wait(full + c % p.stages, (uint32_t)(c / p.stages) & 1u, p.timeout_ns);
     }
 }
 
