@@ -20,8 +20,8 @@
 //     C (64 rows x N) = A (64 rows x n) B (n x N),  N <= 256 sources,
 // real-split with re/im interleaved along K exactly as in tcsweep.cu; A (the
 // packed invT page) and B (the packed right-hand side) stream through a
-// 4-stage bulk-copy ring into kind::tf32 MMAs of N columns, the accumulator
-// sits in tensor memory.  After the MMAs each CTA writes its rows of the new
+// bulk-copy ring of 2 to 5 stages (ck_ring) into kind::tf32 MMAs of N columns,
+// the accumulator sits in tensor memory.  After the MMAs each CTA writes its rows of the new
 // state (re and im planes, rows fastest) and of u, meets its group on a
 // counter barrier, evaluates the next step's stencil for its rows (the
 // neighbour rows come from L2) into the packed B chunks, and meets the group
@@ -40,19 +40,42 @@ namespace wust {
 
 constexpr int kCkThreads = 512;
 constexpr int kCkWarps = kCkThreads / 32;
-constexpr int kCkMinStages = 4, kCkMaxStages = 10;
+constexpr int kCkRingChunks = 4, kCkMaxStages = 5;               // room of the ring: K chunks of kCkMaxN sources
 constexpr int kCopyTid = 96, kCopyBTid = 128;                    // the ring's copy threads, of A and of B (lanes 0)
 constexpr int kCkMaxN = 256;                                     // sources per launch (MMA N)
 constexpr int kCkRowsPerChunk = 16;                              // complex rows per K chunk (TF32)
 constexpr int kCkRowsPerChunk16 = 32;                            // complex rows per K chunk (BF16)
 constexpr int kCkMaxChunks = 148;
 constexpr size_t kCkBSlot = (size_t)kCkMaxN * tc::kChunkBytes;   // 32 KB
-constexpr size_t kCkSmemRing = (size_t)kCkMinStages * (tc::kAChunk + kCkBSlot);
+constexpr size_t kCkSmemRing = (size_t)kCkRingChunks * (tc::kAChunk + kCkBSlot);
 constexpr size_t kCkSmemHalo = 2 * kCkMaxN * sizeof(float2);
 constexpr size_t kCkSmemW = 3 * 64 * sizeof(float2);
 constexpr size_t kCkSmem = kCkSmemRing + kCkSmemHalo + kCkSmemW + 256;
-static_assert((size_t)kCkMinStages * tc::kChunkBytes >= 64 * sizeof(float2), "B stages hold the staged state");
 static_assert(kCkSmem <= 232448, "shared memory of one CTA");
+
+// The ring of a launch of N sources: as many stages as the shared memory holds,
+// and K chunks per stage so that a stage's products take about as long as its
+// share of the waits, commits and copies: a 16-row chunk of 256 sources is 512
+// cycles of MMAs, of 128 sources 256, of 16 (the boundary chain) 192.
+// Measured with 4 / 2 / 1 chunks per stage against 1: 288^2 Hessian product
+// 26.9 against 28.5 ms, 437 x 401 solve 16.6 against 17.9; two at N = 256 (two
+// stages left in the ring): 552^2 gradient 70.5 against 68.3.
+struct CkRing { int per_stage, stages; };
+constexpr CkRing ck_ring(int N) {
+    const int per = N <= 64 ? 4 : N <= 128 ? 2 : 1;
+    return CkRing{per, (int)(kCkSmemRing / (per * (tc::kAChunk + (size_t)N * tc::kChunkBytes)))};
+}
+constexpr bool ck_rings_hold() {
+    for (int N = 8; N <= kCkMaxN; N += 8) {
+        const CkRing r = ck_ring(N);
+        // the B stages hold the staged state between a step's MMAs and the next step's copies
+        if (r.stages < 2 || r.stages > kCkMaxStages ||
+            (size_t)r.stages * r.per_stage * tc::kChunkBytes < 64 * sizeof(float2))
+            return false;
+    }
+    return true;
+}
+static_assert(ck_rings_hold(), "a ring of two stages at least, whose B stages hold the staged state");
 
 __host__ __device__ constexpr int ceil_div8(int x) { return (x + 7) / 8 * 8; }
 
@@ -1006,15 +1029,9 @@ static void set_bounds(ChunkParams &p, int C, bool adjoint, int half) {
 static void ck_launch(ChunkParams &p, bool adjoint, bool bf16, int pass, int groups, cudaStream_t st) {
     if (groups <= 0) return;
     p.pass = pass;
-    // As many stages as the shared memory holds, and K chunks per stage so that
-    // a stage's products take about as long as its share of the waits, commits
-    // and copies: a 16-row chunk of 256 sources is 512 cycles of MMAs, of 128
-    // sources 256, of 16 (the boundary chain) 192.  Measured with 4 / 2 / 1
-    // chunks per stage against 1: 288^2 Hessian product 26.9 against 28.5 ms,
-    // 437 x 401 solve 16.6 against 17.9; two at N = 256 (two stages left in the
-    // ring): 552^2 gradient 70.5 against 68.3.
-    p.per_stage = p.N <= 64 ? 4 : p.N <= 128 ? 2 : 1;
-    p.stages = std::min<int>(kCkMaxStages, (int)(kCkSmemRing / (p.per_stage * (tc::kAChunk + (size_t)p.N * tc::kChunkBytes))));
+    const CkRing ring = ck_ring(p.N);
+    p.per_stage = ring.per_stage;
+    p.stages = ring.stages;
     WUST_CUDA(cudaMemsetAsync(p.group_ctr, 0, sizeof(unsigned) * groups, st));
     void *args[] = {&p};
     const dim3 grid(groups * p.mt), block(kCkThreads);
