@@ -6,20 +6,23 @@
 // of it, and latency-critical callers for which the implicit device
 // synchronization of cudaMalloc/cudaFree is not acceptable.  For them,
 // wust_decomp_block_lu_noalloc runs the same factorization kernel as
-// wust_decomp_block_lu, but its scratch (working page, row/column panels,
-// grid-barrier word and status words) lives in one file-scope __device__
-// array that is part of the loaded module: every GPU that loads the library
-// holds kNoallocScratchBytes for it until the process exits.
+// wust_decomp_block_lu, but its scratch (panels or working pages, grid-barrier
+// word and status words) lives in one file-scope __device__ array that is part
+// of the loaded module: every GPU that loads the library holds
+// kNoallocScratchBytes for it until the process exits.
 //
 // Limits and sharing rules:
 //   * Ny <= WUST_NOALLOC_MAX_NY (1024); larger grids are rejected with
 //     WUST_ERR_INVALID_INPUT before any device work.
 //   * All calls on a device share the one array, which keeps whatever the
-//     last call left in it.  The launcher clears the barrier and status words
-//     at the start of every call; the working page and panels are fully
-//     rewritten before they are read.  Two calls whose work overlaps on the
-//     GPU (different streams, or host threads without ordering) race on the
-//     array and corrupt each other's results; callers must serialize them.
+//     last call left in it.  Pages of up to kFlowMaxTiles tiles an edge take
+//     the dataflow kernel, whose readers poll the panels' words for tags that
+//     start at 1 in every call: its launcher clears all of them, or words of
+//     the call before would be taken for data.  For larger pages it clears
+//     the barrier and status words; those working pages are fully rewritten
+//     before they are read.  Two calls whose work overlaps on the GPU
+//     (different streams, or host threads without ordering) race on the array
+//     and corrupt each other's results; callers must serialize them.
 //   * Every call looks up the array's device address (cudaGetSymbolAddress)
 //     with the caller's device current, so a device reset between calls (a
 //     host such as MATLAB can reset the GPU, which reloads the module,
@@ -34,6 +37,9 @@ namespace wust {
 constexpr int kNoallocMaxNy = WUST_NOALLOC_MAX_NY;
 // Scratch of factor_launch for Ny = kNoallocMaxNy, rounded up to 256 bytes.
 constexpr size_t kNoallocScratchBytes = (factor_scratch_bytes_for(kNoallocMaxNy) + 255) / 256 * 256;
+// the need is not monotonic in Ny: the dataflow kernel's, at its largest page, is that of a page beyond it
+static_assert(factor_scratch_bytes_for(kFlowMaxTiles * kFactorTile + 2) <= kNoallocScratchBytes,
+              "the static scratch holds the largest page of the dataflow kernel");
 
 static __device__ __align__(256) unsigned char g_factor_scratch[kNoallocScratchBytes];
 
