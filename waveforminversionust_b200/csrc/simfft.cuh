@@ -119,10 +119,6 @@ __device__ __forceinline__ float2 turn2(float2 a) { return make_float2(a.y, -a.x
 template <int R>
 struct Dft;
 template <>
-struct Dft<1> {
-    static __device__ __forceinline__ void run(float2 (&)[1]) {}
-};
-template <>
 struct Dft<2> {
     static __device__ __forceinline__ void run(float2 (&x)[2]) {
         const float2 t = x[0];

@@ -115,9 +115,6 @@ __device__ __forceinline__ void bulk_g2s_hint(void *dst, const void *src, uint32
         "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(pol)
         : "memory");
 }
-__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ uint64_t smem_desc(const void *p) {
     uint64_t d = 0;
     d |= (uint64_t)((smem_u32(p) >> 4) & 0x3FFF);                 // start address
