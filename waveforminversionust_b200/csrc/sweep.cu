@@ -284,6 +284,8 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
     using Sh = SweepShape<ADJ, RW, NSW>;
     constexpr int TR = Sh::TR, NS = Sh::NS, NSP = Sh::NSP, HS = NS / 2, PS = Sh::PS, ITEMS = Sh::ITEMS;
     constexpr int SK = Sh::SK, INN = Sh::INN;
+    // a last stage of K that is not full: all of it with the entries beyond n as zeros, or a loop over what is left
+    constexpr bool kWholeTail = RW * NSW <= 16;
     extern __shared__ __align__(128) uint8_t cs_smem[];
     const int ny = p.ny, nx = p.nx, n = p.n, ldc = Sh::ldc(ny), kper = Sh::kper(n);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -555,43 +557,53 @@ __global__ void __launch_bounds__(CT, 1) sweep_cluster_kernel(const __grid_const
                 const float2 *Ar[RW];
 #pragma unroll
                 for (int x = 0; x < RW; ++x) Ar[x] = column(trow(x) - Sh::WR * warp, g * SK + 1) + part;
-                auto product = [&](int kk) {
+                auto product = [&](int kk, bool in) {
                     float2 b[NSW];
                     load_pairs(b, Bs + kk * NSP);
 #pragma unroll
+                    for (int y = 0; y < NSW; ++y) b[y] = in ? b[y] : f2(0.f, 0.f);
+#pragma unroll
                     for (int x = 0; x < RW; ++x) {
-                        const float2 a = Ar[x][kk];
+                        const float2 a = in ? Ar[x][kk] : f2(0.f, 0.f);
 #pragma unroll
                         for (int y = 0; y < NSW; ++y) cfma_conj(acc[x][y], a, b[y]);
                     }
                 };
                 if (left >= SK) {
 #pragma unroll
-                    for (int kk = 0; kk < SK; kk += 8) product(kk);
+                    for (int kk = 0; kk < SK; kk += 8) product(kk, true);
+                } else if constexpr (kWholeTail) {
+#pragma unroll
+                    for (int kk = 0; kk < SK; kk += 8) product(kk, kk < left - part);
                 } else {
 #pragma unroll 1
-                    for (int kk = 0; kk < left - part; kk += 8) product(kk);
+                    for (int kk = 0; kk < left - part; kk += 8) product(kk, true);
                 }
             } else {
                 const float2 *Bs = X + (size_t)(k_own + g * SK) * NSP + tsrc;
                 const float2 *A0 = column(0, r0 + 1) + trow(0), *A1 = column(1, r0 + 1) + trow(0);   // SK is even
-                auto product = [&](int kk) {
+                auto product = [&](int kk, bool in) {
                     const float2 *Ak = (kk & 1 ? A1 : A0) + (kk >> 1) * INN;
                     float2 b[NSW];
                     load_pairs(b, Bs + kk * NSP);
 #pragma unroll
+                    for (int y = 0; y < NSW; ++y) b[y] = in ? b[y] : f2(0.f, 0.f);
+#pragma unroll
                     for (int x = 0; x < RW; ++x) {
-                        const float2 a = Ak[16 * x];
+                        const float2 a = in ? Ak[16 * x] : f2(0.f, 0.f);
 #pragma unroll
                         for (int y = 0; y < NSW; ++y) cfma(acc[x][y], a, b[y]);
                     }
                 };
                 if (left >= SK) {
 #pragma unroll
-                    for (int kk = 0; kk < SK; ++kk) product(kk);
+                    for (int kk = 0; kk < SK; ++kk) product(kk, true);
+                } else if constexpr (kWholeTail) {
+#pragma unroll
+                    for (int kk = 0; kk < SK; ++kk) product(kk, kk < left);
                 } else {
 #pragma unroll 1
-                    for (int kk = 0; kk < left; ++kk) product(kk);
+                    for (int kk = 0; kk < left; ++kk) product(kk, true);
                 }
             }
         }
