@@ -952,17 +952,17 @@ def main():
     else:
         flop = fl["factor"]
         achieved = flop / (head["factor_ms"] * 1e-3) / 1e12
-        kname = ("ns_factor_kernel + factor_kernel (Newton-Schulz Schur inverses, Gauss-Jordan pages)"
-                 if args.precision == "tf32-refined" else "factor_kernel (Schur recursion + Gauss-Jordan inverses)")
+        kname = ("ns_factor_kernel + factor_flow_kernel (Newton-Schulz Schur inverses, Gauss-Jordan pages)"
+                 if args.precision == "tf32-refined" else "factor_flow_kernel (Schur recursion + Gauss-Jordan inverses)")
     # DRAM bytes of one sweep pair of the dominant kernel (its six launches),
     # measured with ncu (dram__bytes_read.sum + dram__bytes_write.sum, one
-    # pass) at 552^2 with 256 sources: TF32 pair 12.48 GB read + 1.19 GB
+    # pass) at 552^2 with 256 sources: TF32 pair 12.48 GB read + 1.28 GB
     # written, BF16 correction pair 8.27 + 1.16 GB; weighted by the step's
     # 2 TF32 pairs and (pairs - 2) BF16 pairs
     traffic = None
     if flop == fl["apply"] and args.precision == "tf32-refined" and WORKLOAD == "config2":
         n_pairs = max(head["sweeps_per_step"], 2.0)
-        traffic = (2 * 13.67e9 + (n_pairs - 2) * 9.42e9) / n_pairs
+        traffic = (2 * 13.76e9 + (n_pairs - 2) * 9.43e9) / n_pairs
     roofline = dict(kernel=kname, bound="tensor", achieved=achieved, peak=peak_tf, unit="TFLOP/s",
                     frac=achieved / peak_tf, peak_source=peak_src, traffic=traffic,
                     traffic_unit="bytes per launch (ncu)", hbm_gbs_achieved=(

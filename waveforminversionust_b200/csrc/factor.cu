@@ -876,7 +876,7 @@ void factor_launch(const Coefs<float2> &co, float2 *invT, void *scratch, size_t 
     if (first < 0 || first >= last || last > co.nx) fail(WUST_ERR_RUNTIME, "factor page range [%d, %d) invalid", j0, j1);
     const unsigned long long timeout_ns = (unsigned long long)(timeout_s * 1e9);
     int *tail = nullptr;
-    // One tile per CTA: the dataflow kernel (552 pages of 552^2 in 76 ms
+    // One tile per CTA: the dataflow kernel (552 pages of 552^2 in 73 ms
     // against 169, 64 of 64^2 in 1.4 against 3.5).  Larger pages, or a grid
     // capped below the tiles, take the kernel whose CTAs walk over several
     // tiles between grid barriers.

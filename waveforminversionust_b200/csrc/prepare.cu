@@ -353,6 +353,8 @@ __global__ void __launch_bounds__(kFoldThreads, NB <= 2 ? 2 : 1) dtft_fold_kerne
 
 // Whether the samples are evenly spaced to rounding: within 1e-11 of a step
 // (the phase of a frequency below Nyquist is then off by less than 1e-10).
+// Times more than some 45,000 steps from zero are not, by their own rounding in
+// 64 bits: such a record takes the general kernel.
 static bool evenly_spaced(const double *t, int nt, double &h) {
     h = (t[nt - 1] - t[0]) / (nt - 1);
     for (int i = 0; i < nt; ++i)

@@ -179,9 +179,10 @@ __global__ void sim_decimate_kernel(const float *__restrict__ in, int nt, int n_
 // A step reads and writes 22 planes per transmitter (the transforms of a
 // library each pass over their planes two or three times more, and the
 // pointwise kernels between them over all of them again: 50).  What bounds a
-// tile is the latency of its phases (loads, stages, barriers: 0.4 of the issue
-// slots, 15 % of the memory's rate), hence the three tiles an SM and the loads
-// in batches.  Microseconds per step, library transforms -> here:
+// tile is the latency of its phases (loads, stages, barriers: 0.41 to 0.46 of
+// the issue slots at 288^2 x 64; 30 % of the memory's rate at 552^2), hence the
+// three tiles an SM and the loads in batches.  Microseconds per step, library
+// transforms -> here:
 //   552^2, 64 transmitters         1126 -> 870
 //   288^2, 64                       343 -> 274
 //   1024 x 800, 4                   218 -> 172

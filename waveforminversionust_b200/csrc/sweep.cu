@@ -219,8 +219,8 @@ static void launch_gemm(const float2 *A, const float2 *B, size_t ldb, float2 *C,
 // exchange - barrier - stencil.  The cluster barrier is the hardware's, and
 // every thread of the cluster reaches it; there is no other wait.
 // Measured, us per column step before (two launches) -> now: 552^2 x 256 H
-// 35 -> 26, H^H 43 -> 27; 224^2 x 32 18 -> 4.0, 20 -> 5.1; 64^2 x 6 9.4 -> 2.1,
-// 9.9 -> 2.9.
+// 35 -> 23, H^H 44 -> 25; 224^2 x 32 18 -> 3.9, 20 -> 4.9; 64^2 x 6 9.3 -> 1.8,
+// 8.6 -> 2.6.
 // ---------------------------------------------------------------------------
 constexpr int CT = 256, CW = CT / 32;    // threads, warps
 constexpr int kCsMaxCl = 8;
