@@ -55,8 +55,8 @@ def test_factor_reports_a_singular_page(ny, row):
     assert np.array_equal(decompBlockLU(*_device(coefs)).cpu().numpy(), good)
 
 
-# one interior row; odd and even column lengths (the parity of a page column's first byte); the largest column of the
-# widest shape, the first beyond it, and the first that takes a launch per column step
+# one interior row; odd and even column lengths (the parity of a page column's first byte); columns that take a launch
+# per column step (H beyond 570 rows, H^H beyond 642; the shapes of the one launch are in test_gpu_sweep_cluster.py)
 @pytest.mark.parametrize("ny,nx,S", [(3, 3, 1), (3, 5, 3), (18, 7, 5), (19, 6, 2), (64, 9, 13), (97, 8, 1), (194, 5, 40),
                                      (195, 5, 41), (578, 4, 30), (642, 4, 20), (770, 4, 3), (771, 4, 3)])
 @pytest.mark.parametrize("adjoint", [False, True])
