@@ -138,8 +138,11 @@ def workspace(need: int, stream):
     if not 0 < need <= WORKSPACE_LIMIT or not isinstance(stream, torch.cuda.Stream):
         return None, None
     try:
-        with torch.cuda.stream(stream):
+        if stream == torch.cuda.current_stream():
             block = torch.empty(need + 256, dtype=torch.uint8, device="cuda")
+        else:
+            with torch.cuda.stream(stream):
+                block = torch.empty(need + 256, dtype=torch.uint8, device="cuda")
     except torch.OutOfMemoryError:
         return None, None
     return block, C.c_void_p(-(-block.data_ptr() // 256) * 256)
