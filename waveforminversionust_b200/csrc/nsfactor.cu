@@ -319,6 +319,7 @@ __global__ void __launch_bounds__(kNsThreads, 1) ns_factor_kernel(NsParams p) {
             const uint8_t *ab = Apack + ((size_t)mt * p.kc + c0) * tc::kAChunk;
             const uint8_t *bb = Bpack + ((size_t)nb * p.kc + c0) * kBChunkNs;
             bool good = true;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the copies land where partial tiles were staged
             for (int c = 0; c < nch && good; ++c) {
                 const uint32_t s = u_issue % kStages, f = u_issue / kStages;
                 if (f >= 1 && !tc::mbar_wait(&empty[s], (f - 1) & 1u, p.timeout_ns)) {

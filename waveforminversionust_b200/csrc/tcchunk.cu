@@ -651,6 +651,7 @@ __global__ void __launch_bounds__(kCkThreads, 1) tc_chunk_kernel(const __grid_co
     };
     // B: every stage of a step
     auto copies_b = [&]() {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the copies land where the state was staged
         const uint8_t *src = bg;
         for (int q = 0; q < kc; q += G) {
             if (!stage_free()) {

@@ -350,6 +350,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1) tc_sweep_kernel(SweepParams 
 
         // ---- B of this step -> shared memory; MMAs (one thread) -------------
         if (tid == 0) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the copies land where the reductions had their scratch
             for (int q = 0; q < nch; ++q) {
                 tc::mbar_expect_tx(&full[q], kBChunk);
                 tc::bulk_g2s(sB + (size_t)q * kBChunk, bg + (size_t)(c0 + q) * kBChunk, kBChunk, &full[q]);
