@@ -220,8 +220,8 @@ static void launch_gemm(const float2 *A, const float2 *B, size_t ldb, float2 *C,
 // exchange - barrier - stencil.  The cluster barrier is the hardware's, and
 // every thread of the cluster reaches it; there is no other wait.
 // Measured, us per column step before (two launches) -> now: 552^2 x 256 H
-// 35 -> 23, H^H 44 -> 25; 224^2 x 32 18 -> 3.9, 20 -> 4.9; 64^2 x 6 9.3 -> 1.8,
-// 8.6 -> 2.6.
+// 35 -> 23, H^H 44 -> 25; 224^2 x 32 18 -> 3.7, 20 -> 4.9; 64^2 x 6 9.3 -> 1.8,
+// 8.6 -> 2.5.
 // ---------------------------------------------------------------------------
 constexpr int CT = 256, CW = CT / 32;    // threads, warps
 constexpr int kCsMaxCl = 8;
